@@ -1635,15 +1635,35 @@ int tpo_sensitivity_filter(const tpo_grid *g, double rmin, const double *rho, co
 }
 
 // ------------------------------------------------------------------ OC
-static dim3 oc_grid(size_t n) { return flat_grid(n, OC_THREADS, 148 * 4); }
+// One cluster up to the elements its threads hold in registers: 8 CTAs finish
+// a pass (barrier included) before a cooperative grid has exchanged its sums.
+// Beyond that one element per thread and CTA until every SM has a CTA.
+static constexpr int kOcClusterElems = kClusterCtas * OC_THREADS * OC_EPT;
+static int oc_ctas(size_t n) {
+  return (int)std::min<size_t>((n + OC_THREADS - 1) / OC_THREADS, (size_t)sm_count());
+}
+static bool oc_held(size_t n) {
+  return n <= kOcClusterElems || n <= (size_t)oc_ctas(n) * OC_THREADS * OC_EPT;
+}
+
+struct OcWs {
+  GridBar *bar;
+  double *part, *sbuf;
+  size_t bytes;
+};
+static OcWs carve_oc(void *base, size_t n) {
+  Carve cv(base);
+  OcWs w{};
+  w.bar = cv.take<GridBar>(1);
+  w.part = cv.take<double>(2 * OC_NL * (size_t)std::max(sm_count(), 1));
+  w.sbuf = cv.take<double>(n);
+  w.bytes = cv.off;
+  return w;
+}
 
 size_t tpo_oc_workspace_bytes(const tpo_grid *g) {
   if (check_grid(g)) return 0;
-  const dim3 gr = oc_grid((size_t)g->nelx * g->nely);
-  Carve cv(nullptr);
-  cv.take<OcCtl>(1);
-  cv.take<double>(2 * (size_t)gr.x);
-  return cv.off;
+  return carve_oc(nullptr, (size_t)g->nelx * g->nely).bytes;
 }
 
 int tpo_oc_update(const tpo_grid *g, double volfrac, double move, const double *rho_in,
@@ -1654,19 +1674,21 @@ int tpo_oc_update(const tpo_grid *g, double volfrac, double move, const double *
   if (!rho_in || !dc || !rho_out || !ws) return fail(TPO_ERR_ARGS, "NULL pointer argument");
   if (!aligned(ws, kAlign)) return fail(TPO_ERR_ARGS, "misaligned workspace");
   if (ws_bytes < tpo_oc_workspace_bytes(g)) return fail(TPO_ERR_WORKSPACE, "workspace too small");
-  const size_t n = (size_t)g->nelx * g->nely;
-  const dim3 gr = oc_grid(n);
+  int n = g->nelx * g->nely;
   cudaStream_t st = static_cast<cudaStream_t>(s);
-  Carve cv(ws);
-  OcCtl *ctl = cv.take<OcCtl>(1);
-  double *part = cv.take<double>(2 * (size_t)gr.x);
-  k_oc_init<<<1, 1, 0, st>>>(ctl);
-  TPO_CK_LAUNCH();
-  for (int i = 0; i < OC_MAX_STEPS; ++i) {
-    k_oc_step<<<gr, OC_THREADS, 0, st>>>((int)n, volfrac, move, rho_in, dc, dv, part, ctl);
-    TPO_CK_LAUNCH();
+  OcWs w = carve_oc(ws, (size_t)n);
+  if (n <= kOcClusterElems) {
+    k_oc_cluster<true><<<kClusterCtas, OC_THREADS, 0, st>>>(n, volfrac, move, rho_in, dc, dv,
+                                                            w.sbuf, rho_out, result_out);
+  } else {
+    TPO_CK(cudaMemsetAsync(w.bar, 0, sizeof(GridBar), st));
+    void *args[] = {&n, &volfrac, &move, &rho_in, &dc, &dv, &w.sbuf, &rho_out, &result_out,
+                    &w.bar, &w.part};
+    const void *kern = oc_held((size_t)n) ? (const void *)k_oc_grid<true>
+                                          : (const void *)k_oc_grid<false>;
+    TPO_CK(cudaLaunchCooperativeKernel(kern, dim3(oc_ctas((size_t)n)), dim3(OC_THREADS), args, 0,
+                                       st));
   }
-  k_oc_final<<<gr, OC_THREADS, 0, st>>>((int)n, move, rho_in, dc, dv, rho_out, ctl, result_out);
   TPO_CK_LAUNCH();
   return TPO_OK;
 }

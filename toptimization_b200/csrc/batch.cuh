@@ -255,66 +255,22 @@ __global__ void __launch_bounds__(S_THREADS) kb_sens(const BJob *jobs, int nj, c
                   loc % J.gx, loc / J.gx, J.gx * J.gy, loc);
 }
 
-// OC update of one design per CTA (reference optimizer/oc.py:21-93, same
-// rules as k_oc_step / k_oc_final): bisection on lambda in [0, 1e9], at most
-// OC_MAX_STEPS midpoints, stop when (hi - lo) / (hi + lo) < 1e-4; the density
-// is updated in place with the last midpoint evaluated. One CTA loops over the
-// steps, so the whole bisection is one launch for every design of the batch.
-constexpr int OCB_THREADS = 1024;
-__global__ void __launch_bounds__(OCB_THREADS) kb_oc(BDesign *ds, int n) {
-  if ((int)blockIdx.x >= n) return;
-  BDesign &D = ds[blockIdx.x];
+// OC update (oc_run, design.cuh), one cluster per design, in place. s goes to
+// D.dc, which the dc filter has read. A design's cluster is the same alone and
+// in any mix, so its sums are. One CTA per design and one midpoint per pass
+// took 7 ms for a 512x512 design; eight CTAs and seven midpoints per pass take
+// about 0.1 ms.
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(OC_THREADS, 1)
+    kb_oc(BDesign *ds, int n) {
+  const int slot = (int)blockIdx.x / kClusterCtas;
+  if (slot >= n) return;
+  BDesign &D = ds[slot];
   if (!D.active || D.phase != PH_POST) return;
-  __shared__ double red[2][OCB_THREADS / 32];
-  __shared__ double res[2];
-  const int ne = D.nx * D.ny;
-  const double *rho = D.rho;  // updated in place at the end
-  const double *__restrict__ dcf = D.dc_filt;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  double lo = 0.0, hi = 1e9, lam = 0.5 * (0.0 + 1e9), last = 0.0, chg = 0.0, vol = 0.0;
-  int steps = 0;
-  for (;;) {
-    double sum = 0.0, mx = 0.0;
-    for (int e = threadIdx.x; e < ne; e += OCB_THREADS) {
-      const double r = rho[e];
-      const double nw = oc_candidate(r, dcf[e], 1.0, lam, D.move);
-      sum += nw;
-      mx = fmax(mx, fabs(nw - r));
-    }
-    sum = warp_sum(sum);
-    mx = warp_max(mx);
-    if (lane == 0) {
-      red[0][wid] = sum;
-      red[1][wid] = mx;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = red[0][0], m = red[1][0];
-      for (int w = 1; w < OCB_THREADS / 32; ++w) {
-        t += red[0][w];
-        m = fmax(m, red[1][w]);
-      }
-      res[0] = t;
-      res[1] = m;
-    }
-    __syncthreads();
-    last = lam;
-    chg = res[1];
-    vol = res[0] / ne;
-    steps += 1;
-    if (vol > D.volfrac) lo = lam; else hi = lam;
-    if ((hi - lo) / (hi + lo + 1e-30) < 1e-4 || steps >= OC_MAX_STEPS) break;
-    lam = 0.5 * (lo + hi);
-    __syncthreads();  // res[] is rewritten by the next step
-  }
-  for (int e = threadIdx.x; e < ne; e += OCB_THREADS)
-    D.rho[e] = oc_candidate(rho[e], dcf[e], 1.0, last, D.move);
-  if (threadIdx.x == 0) {
-    D.scal[1] = chg;
-    D.scal[2] = vol;
-    D.scal[3] = last;
-    D.scal[4] = (double)steps;
-  }
+  __shared__ typename ClusterTeam<OC_NL>::Shared ts;
+  __shared__ OcShared sh;
+  ClusterTeam<OC_NL> team(ts);
+  oc_run<false>(team, D.nx * D.ny, D.volfrac, D.move, D.rho, D.dc_filt, nullptr, D.dc, D.rho,
+                D.scal + 1, sh);
 }
 
 // one thread per slot: history row, iteration count, stop rule

@@ -276,7 +276,7 @@ int batch_suffix(tpo_batch *b, cudaStream_t st) {
   kb_filter<<<b->nctas[BK_FILTER], F_THREADS, b->filter_smem, st>>>(
       jobs_of(b, BK_FILTER), b->njobs[BK_FILTER], b->d_designs, 1);
   TPO_CK_LAUNCH();
-  kb_oc<<<b->n_slots, OCB_THREADS, 0, st>>>(b->d_designs, b->n_slots);
+  kb_oc<<<b->n_slots * kClusterCtas, OC_THREADS, 0, st>>>(b->d_designs, b->n_slots);
   TPO_CK_LAUNCH();
   kb_finish<<<cdiv(b->n_slots, 128), 128, 0, st>>>(b->d_designs, b->n_slots, b->d_status,
                                                    b->d_flag + 2);

@@ -119,12 +119,10 @@ struct OuterCtl {
   int32_t max_outer;  // residual evaluations allowed (then TPO_SOLVE_MAX_ITER)
 };
 
-struct OcCtl {
-  double lo, hi, mid;
-  double last_mid, change, vol;
-  int32_t steps, done;
-  uint32_t counter;
-  int32_t pad;
+// Arrival counter of a cooperative grid's barriers, zeroed before the launch.
+struct GridBar {
+  uint32_t arrived;
+  uint32_t err;  // nonzero: a bounded wait ran out
 };
 
 struct SumCtl {
@@ -196,5 +194,149 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double *part, uint3
 }
 
 __device__ __forceinline__ bool finite(double x) { return isfinite(x); }
+
+// ---------------------------------------------------------------- co-resident CTAs
+// Kernels that iterate on the device synchronise their CTAs in one of two
+// ways: a thread-block cluster (its barrier, sums exchanged through
+// distributed shared memory) or a cooperative launch (a counter in global
+// memory). Both offer the same deterministic all-reduce: every CTA gets the
+// totals, summed in CTA order, in its shared memory (valid until the next
+// call; nullptr when a bounded wait ran out).
+
+__device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// Waits until the counter reaches `target`; about ten seconds at most, after
+// which *err is set and false returned.
+__device__ __forceinline__ bool wait_count(const uint32_t *p, uint32_t target, uint32_t *err) {
+  for (long long i = 0; i < (1ll << 24); ++i) {
+    if (ld_acquire(p) >= target) return true;
+    if (i > 64) __nanosleep(64);
+    if ((i & 1023) == 1023 && ld_acquire(err)) return false;
+  }
+  atomicExch(err, 1u);
+  return false;
+}
+
+// CTA part of the all-reduce: totals of NV per-thread values over the CTA,
+// value k in lane 0 of warp k (blockDim.x >= 32 NV; sm holds NV * 32 doubles).
+template <int NV, unsigned MAXMASK>
+__device__ __forceinline__ double cta_reduce(const double (&v)[NV], double *sm) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const double t = ((MAXMASK >> k) & 1u) ? warp_max(v[k]) : warp_sum(v[k]);
+    if (lane == 0) sm[k * 32 + wid] = t;
+  }
+  __syncthreads();
+  double t = 0.0;
+  if (wid < NV) {
+    t = lane < nw ? sm[wid * 32 + lane] : 0.0;
+    t = ((MAXMASK >> wid) & 1u) ? warp_max(t) : warp_sum(t);
+  }
+  return t;
+}
+
+constexpr int kClusterCtas = 8;  // portable cluster size
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ double ld_cluster(const double *sm, uint32_t rank) {
+  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(sm)), b;
+  double v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(b) : "memory");
+  return v;
+}
+
+// One cluster of kClusterCtas CTAs.
+template <int NVMAX> struct ClusterTeam {
+  struct Shared {
+    double sm[NVMAX * 32];
+    double mine[2][NVMAX];  // this CTA's totals, by parity of the call
+    double tot[NVMAX];
+  };
+  Shared &s;
+  int calls = 0;
+  __device__ explicit ClusterTeam(Shared &sh) : s(sh) {}
+  __device__ int rank() const { return (int)cluster_rank(); }
+  __device__ int size() const { return kClusterCtas; }
+  template <int NV, unsigned MAXMASK = 0u>
+  __device__ const double *reduce(const double (&v)[NV]) {
+    const double t = cta_reduce<NV, MAXMASK>(v, s.sm);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, b = calls++ & 1;
+    if (wid < NV && lane == 0) s.mine[b][wid] = t;
+    cluster_sync();
+    if (wid < NV) {
+      double x = lane < kClusterCtas ? ld_cluster(&s.mine[b][wid], lane) : 0.0;
+      x = ((MAXMASK >> wid) & 1u) ? warp_max(x) : warp_sum(x);
+      if (lane == 0) s.tot[wid] = x;
+    }
+    __syncthreads();
+    return s.tot;
+  }
+  // no CTA leaves while another may still read its shared memory
+  __device__ void leave() { cluster_sync(); }
+};
+
+// A cooperative launch: part holds 2 * NVMAX * size() doubles.
+template <int NVMAX> struct GridTeam {
+  struct Shared {
+    double sm[NVMAX * 32];
+    double tot[NVMAX];
+    int ok;
+  };
+  Shared &s;
+  GridBar *bar;
+  double *part;
+  int calls = 0;
+  __device__ GridTeam(Shared &sh, GridBar *b, double *p) : s(sh), bar(b), part(p) {}
+  __device__ int rank() const { return (int)blockIdx.x; }
+  __device__ int size() const { return (int)gridDim.x; }
+  template <int NV, unsigned MAXMASK = 0u>
+  __device__ const double *reduce(const double (&v)[NV]) {
+    const double t = cta_reduce<NV, MAXMASK>(v, s.sm);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, n = size();
+    if (n == 1) {
+      if (wid < NV && lane == 0) s.tot[wid] = t;
+      __syncthreads();
+    } else {
+      double *pp = part + (size_t)(calls & 1) * NVMAX * n;
+      if (wid < NV && lane == 0) {
+        pp[wid * n + rank()] = t;
+        __threadfence();
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        atomicAdd(&bar->arrived, 1u);
+        s.ok = wait_count(&bar->arrived, (uint32_t)(calls + 1) * n, &bar->err) ? 1 : 0;
+      }
+      __syncthreads();
+      if (!s.ok) return nullptr;
+      if (wid < NV) {
+        double x = 0.0;
+        for (int i = lane; i < n; i += 32) {
+          const double y = __ldcg(pp + wid * n + i);
+          x = ((MAXMASK >> wid) & 1u) ? fmax(x, y) : x + y;
+        }
+        x = ((MAXMASK >> wid) & 1u) ? warp_max(x) : warp_sum(x);
+        if (lane == 0) s.tot[wid] = x;
+      }
+      __syncthreads();
+    }
+    ++calls;
+    return s.tot;
+  }
+  __device__ void leave() {}
+};
 
 }  // namespace tpo
