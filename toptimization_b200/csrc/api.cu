@@ -19,6 +19,7 @@
 #include "design.cuh"
 #include "pcg.cuh"
 #include "cgstep.cuh"
+#include "cgres.cuh"
 #include "hex3d.cuh"
 #include "stencil.cuh"
 #include "tpo.h"
@@ -843,6 +844,117 @@ int pcg_mixed(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, cons
   return TPO_OK;
 }
 
+// ----------------------------------------------------------------- resident PCG
+// Tiling of the resident solve (k_cgres): the fewest CTAs whose extended tile
+// (tile and halo ring, one node per thread) fits the smallest CTA that keeps
+// them within one per SM; none if 1024 threads do not.
+struct ResPlan {
+  int BX = 0, BY = 0, tx = 0, ty = 0, threads = 0;
+  explicit operator bool() const { return threads > 0; }
+};
+ResPlan res_plan(const tpo_grid *g) {
+  const int cx = g->nelx + 1, cy = g->nely + 1;
+  const int most = std::min(sm_count(), RES_MAX_CTAS);
+  ResPlan p;
+  if ((int64_t)cx * cy > (int64_t)most * RES_MAX_THREADS) return p;
+  for (int T = 256; T <= RES_MAX_THREADS && !p; T += 128) {
+    int64_t best = most + 1;
+    for (int by = 1; by <= std::min(cy, T / 3 - 2); ++by) {
+      const int bx = std::min(cx, T / (by + 2) - 2);
+      if (bx < 1) break;
+      const int64_t tiles = (int64_t)((cx + bx - 1) / bx) * ((cy + by - 1) / by);
+      if (tiles >= best) continue;
+      best = tiles;
+      p.tx = (cx + bx - 1) / bx;
+      p.ty = (cy + by - 1) / by;
+      p.BX = (cx + p.tx - 1) / p.tx;  // the same tiles, evened out
+      p.BY = (cy + p.ty - 1) / p.ty;
+    }
+    if (best <= most) p.threads = std::max(128, ((p.BX + 2) * (p.BY + 2) + 31) / 32 * 32);
+  }
+  return p;
+}
+
+// words of one exchange: two doubles per value, [parity][component][node] and
+// [parity][sum][CTA]; they lie over the vectors w, s and p of the form with one
+// launch per iteration, which this one keeps in registers
+size_t res_words(const tpo_grid *g, const ResPlan &p) {
+  return 4 * (size_t)(g->nelx + 1) * (g->nely + 1) + 6 * (size_t)p.tx * p.ty;
+}
+ResPlan res_plan_in(const tpo_grid *g, const PcgWs &w) {
+  ResPlan p = res_plan(g);
+  const size_t NN = (size_t)(g->nelx + 1) * w.P;
+  if (p && 2 * res_words(g, p) > 10 * NN) p.threads = 0;  // wa, wb, sa, sb, pa
+  return p;
+}
+
+template <int PRE>
+int launch_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const double *f,
+               const uint8_t *fixed, double *u, const PcgWs &w, const ResPlan &p,
+               cudaStream_t st, cudaEvent_t *ev) {
+  const double fn = std::sqrt(c->f_norm_sq);
+  const size_t words = res_words(g, p), nodes = (size_t)(g->nelx + 1) * (g->nely + 1);
+  k_res_init<<<flat_grid(words, 256, sm_count() * 8), 256, 0, st>>>(
+      reinterpret_cast<double2 *>(w.wa), words, w.ctl, (c->tol * fn) * (c->tol * fn), c->max_iter);
+  TPO_CK_LAUNCH();
+  ResArgs a{};
+  a.nx = g->nelx;
+  a.ny = g->nely;
+  a.BX = p.BX;
+  a.BY = p.BY;
+  a.tiles_y = p.ty;
+  a.e_min = g->e_min;
+  a.pen = g->penalty;
+  a.rho = rho;
+  a.f = f;
+  a.fixed = fixed;
+  a.u = u;
+  a.warm = c->warm_start != 0;
+  for (int b = 0; b < 2; ++b)
+    for (int k = 0; k < 2; ++k) a.halo[b][k] = w.wa + 2 * nodes * (2 * b + k);
+  a.sums = w.wa + 8 * nodes;
+  a.ctl = w.ctl;
+  a.withhold1 = g_withhold1.exchange(0);
+  void *args[] = {&a};
+  const void *kern = p.threads <= 512   ? (const void *)k_cgres<PRE, 512>
+                     : p.threads <= 768 ? (const void *)k_cgres<PRE, 768>
+                                        : (const void *)k_cgres<PRE, RES_MAX_THREADS>;
+  if (ev) TPO_CK(cudaEventRecord(ev[0], st));
+  TPO_CK(cudaLaunchCooperativeKernel(kern, dim3(p.tx * p.ty), dim3(p.threads), args,
+                                     res_smem(p.BX, p.BY), st));
+  TPO_CK_LAUNCH();
+  if (ev) TPO_CK(cudaEventRecord(ev[1], st));
+  return TPO_OK;
+}
+
+// Blocking form: the whole solve is two launches.
+template <int PRE>
+int pcg_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const double *f,
+            const uint8_t *fixed, double *u, const PcgWs &w, const ResPlan &p,
+            tpo_solve_result *out, cudaStream_t st) {
+  cudaEvent_t *ev = nullptr;
+  int rc = g_prof_on ? prof_events(1, &ev) : TPO_OK;
+  if (!rc) rc = launch_res<PRE>(g, c, rho, f, fixed, u, w, p, st, ev);
+  if (rc) return rc;
+  PcgCtl fin;
+  TPO_CK(cudaMemcpyAsync(&fin, w.ctl, sizeof(PcgCtl), cudaMemcpyDeviceToHost, st));
+  TPO_CK(cudaStreamSynchronize(st));
+  if (fin.err) return fail(TPO_ERR_TIMEOUT, "an exchange of the resident solve ran out of time");
+  if (ev) {  // profile: the iterations of the launch
+    float ms = 0.f;
+    TPO_CK(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+    g_prof.step_ms += ms;
+    g_prof.step_launches += fin.it;
+    g_prof.step_bytes += (int64_t)fin.it * step_bytes<double>(g).step;
+  }
+  out->status = fin.status == TPO_SOLVE_RUNNING ? TPO_SOLVE_MAX_ITER : fin.status;
+  out->updates = fin.it;
+  out->iters = (out->status == TPO_SOLVE_CONVERGED) ? fin.it : c->max_iter;
+  out->outer_iters = 1;
+  out->rr = fin.rr;
+  return TPO_OK;
+}
+
 // ----------------------------------------------------------------- one-launch PCG
 CgArgs cg_args(const tpo_grid *g, const PcgWs &w) {
   CgArgs a{};
@@ -870,6 +982,8 @@ template <int PRE>
 int pcg_single(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const double *f,
                const uint8_t *fixed, double *u, const PcgWs &w, tpo_solve_result *out,
                cudaStream_t st, double alpha_reg) {
+  if (const ResPlan rp = res_plan_in(g, w))
+    return pcg_res<PRE>(g, c, rho, f, fixed, u, w, rp, out, st);
   const int nx = g->nelx, ny = g->nely, P = w.P;
   const double fn = std::sqrt(c->f_norm_sq);
   const double tol_sq = (c->tol * fn) * (c->tol * fn);
@@ -1066,6 +1180,16 @@ int emit_solve_async(const tpo_grid *g, const tpo_solve_cfg *c, const double *rh
   const bool mixed = c->precision == TPO_PRECISION_MIXED;
   const double fn = std::sqrt(c->f_norm_sq);
   const double tol_sq = (c->tol * fn) * (c->tol * fn);
+  if constexpr (!block) {
+    if (w.single)
+      if (const ResPlan rp = res_plan_in(g, w)) {
+        const int rc = launch_res<PRE>(g, c, rho, f, fixed, u, w, rp, st, nullptr);
+        if (rc) return rc;
+        k_res_result<<<1, 1, 0, st>>>(w.ctl, c->max_iter, out);
+        TPO_CK_LAUNCH();
+        return TPO_OK;
+      }
+  }
   const dim3 sg = flat_grid((size_t)nx * P, 256, sm_count() * 16);
   const int64_t l0 = g_launches.load();
   int n_body = 0;
