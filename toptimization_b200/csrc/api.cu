@@ -846,57 +846,134 @@ int pcg_mixed(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, cons
 
 // ----------------------------------------------------------------- resident PCG
 // Tiling of the resident solve (k_cgres): the fewest CTAs whose extended tile
-// (tile and halo ring, one node per thread) fits the smallest CTA that keeps
-// them within one per SM; none if 1024 threads do not.
+// (tile and halo ring, one node per thread) fits a CTA of T threads. One
+// cluster if 16 CTAs of at most 768 threads hold the grid (its exchange takes
+// about 1 us less, and every further thread adds to the update, the stencil
+// and the sums: at 1024 threads the cooperative form has caught up); otherwise
+// one CTA per SM at most, the smallest T that allows it; none if 1024 threads
+// do not. Measured per iteration, against 13-16 us with one launch each:
+//   cluster:     60x20 1.75 us, 97x41 2.0, 151x49 2.5 (cooperative 2.7, -, 3.0)
+//   cooperative: 160x64 3.1, 200x100 3.7, 400x200 4.9, 460x270 6.3
 struct ResPlan {
   int BX = 0, BY = 0, tx = 0, ty = 0, threads = 0;
+  bool cluster = false;
   explicit operator bool() const { return threads > 0; }
 };
-ResPlan res_plan(const tpo_grid *g) {
+// the tiling with the fewest CTAs for extended tiles of at most T nodes
+int64_t res_tiles(int cx, int cy, int T, ResPlan *p) {
+  int64_t best = INT64_MAX;
+  for (int by = 1; by <= std::min(cy, T / 3 - 2); ++by) {
+    const int bx = std::min(cx, T / (by + 2) - 2);
+    if (bx < 1) break;
+    const int64_t tiles = (int64_t)((cx + bx - 1) / bx) * ((cy + by - 1) / by);
+    if (tiles >= best) continue;
+    best = tiles;
+    p->tx = (cx + bx - 1) / bx;
+    p->ty = (cy + by - 1) / by;
+    p->BX = (cx + p->tx - 1) / p->tx;  // the same tiles, evened out
+    p->BY = (cy + p->ty - 1) / p->ty;
+  }
+  return best;
+}
+ResPlan res_plan(const tpo_grid *g, int cluster_ctas) {
   const int cx = g->nelx + 1, cy = g->nely + 1;
   const int most = std::min(sm_count(), RES_MAX_CTAS);
+  const int64_t nodes = (int64_t)cx * cy;
   ResPlan p;
-  if ((int64_t)cx * cy > (int64_t)most * RES_MAX_THREADS) return p;
-  for (int T = 256; T <= RES_MAX_THREADS && !p; T += 128) {
-    int64_t best = most + 1;
-    for (int by = 1; by <= std::min(cy, T / 3 - 2); ++by) {
-      const int bx = std::min(cx, T / (by + 2) - 2);
-      if (bx < 1) break;
-      const int64_t tiles = (int64_t)((cx + bx - 1) / bx) * ((cy + by - 1) / by);
-      if (tiles >= best) continue;
-      best = tiles;
-      p.tx = (cx + bx - 1) / bx;
-      p.ty = (cy + by - 1) / by;
-      p.BX = (cx + p.tx - 1) / p.tx;  // the same tiles, evened out
-      p.BY = (cy + p.ty - 1) / p.ty;
-    }
-    if (best <= most) p.threads = std::max(128, ((p.BX + 2) * (p.BY + 2) + 31) / 32 * 32);
-  }
+  int64_t tiles = INT64_MAX;
+  if (nodes <= (int64_t)cluster_ctas * RES_CLUSTER_THREADS)
+    for (int T = 128; T <= RES_CLUSTER_THREADS && !p.cluster; T += 32)
+      p.cluster = (tiles = res_tiles(cx, cy, T, &p)) <= cluster_ctas;
+  if (!p.cluster) tiles = INT64_MAX;
+  if (!p.cluster && nodes <= (int64_t)most * RES_MAX_THREADS)
+    for (int T = 256; T <= RES_MAX_THREADS && tiles > most; T += 128)
+      tiles = res_tiles(cx, cy, T, &p);
+  if (tiles <= most)
+    p.threads = std::max(128, ((p.BX + 2) * (p.BY + 2) + 31) / 32 * 32);
   return p;
 }
 
+template <int PRE> const void *res_kernel(const ResPlan &p) {
+  if (p.cluster)
+    return p.threads <= 512 ? (const void *)k_cgres<PRE, 512, true>
+                            : (const void *)k_cgres<PRE, RES_CLUSTER_THREADS, true>;
+  return p.threads <= 512   ? (const void *)k_cgres<PRE, 512, false>
+         : p.threads <= 768 ? (const void *)k_cgres<PRE, 768, false>
+                            : (const void *)k_cgres<PRE, RES_MAX_THREADS, false>;
+}
+void res_launch_config(const ResPlan &p, cudaStream_t st, cudaLaunchConfig_t *lc,
+                       cudaLaunchAttribute *at) {
+  *lc = cudaLaunchConfig_t{};
+  lc->gridDim = dim3(p.tx * p.ty);
+  lc->blockDim = dim3(p.threads);
+  lc->dynamicSmemBytes = res_smem(p.BX, p.BY, p.cluster);
+  lc->stream = st;
+  if (p.cluster) {
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = p.tx * p.ty;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  } else {
+    at->id = cudaLaunchAttributeCooperative;
+    at->val.cooperative = 1;
+  }
+  lc->attrs = at;
+  lc->numAttrs = 1;
+}
+
+// CTAs a cluster of this device can have (16 where a GPC has room, else 8)
+int res_cluster_ctas() {
+  static const int n = [] {
+    int ok = 1;
+    auto allow = [&](const void *k, int threads) {
+      ok &= cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                cudaSuccess;
+      ResPlan p;
+      p.tx = RES_CLUSTER_CTAS;
+      p.ty = 1;
+      p.BX = threads / 22 - 2;
+      p.BY = 20;
+      p.threads = threads;
+      p.cluster = true;
+      cudaLaunchConfig_t lc;
+      cudaLaunchAttribute at;
+      res_launch_config(p, nullptr, &lc, &at);
+      int c = 0;
+      ok &= cudaOccupancyMaxActiveClusters(&c, k, &lc) == cudaSuccess && c > 0;
+    };
+    allow((const void *)k_cgres<TPO_PRECOND_NONE, 512, true>, 512);
+    allow((const void *)k_cgres<TPO_PRECOND_JACOBI, 512, true>, 512);
+    allow((const void *)k_cgres<TPO_PRECOND_NODAL_BLOCK, 512, true>, 512);
+    allow((const void *)k_cgres<TPO_PRECOND_NONE, RES_CLUSTER_THREADS, true>, RES_CLUSTER_THREADS);
+    allow((const void *)k_cgres<TPO_PRECOND_JACOBI, RES_CLUSTER_THREADS, true>,
+          RES_CLUSTER_THREADS);
+    allow((const void *)k_cgres<TPO_PRECOND_NODAL_BLOCK, RES_CLUSTER_THREADS, true>,
+          RES_CLUSTER_THREADS);
+    if (!ok) cudaGetLastError();
+    return ok ? RES_CLUSTER_CTAS : kClusterCtas;
+  }();
+  return n;
+}
+
 // words of one exchange: two doubles per value, [parity][component][node] and
-// [parity][sum][CTA]; they lie over the vectors w, s and p of the form with one
+// [parity][copy][sum][CTA]; they lie over the vectors w, s and p of the form with one
 // launch per iteration, which this one keeps in registers
 size_t res_words(const tpo_grid *g, const ResPlan &p) {
-  return 4 * (size_t)(g->nelx + 1) * (g->nely + 1) + 6 * (size_t)p.tx * p.ty;
+  return 4 * (size_t)(g->nelx + 1) * (g->nely + 1) + 6 * RES_COPIES * (size_t)p.tx * p.ty;
 }
 ResPlan res_plan_in(const tpo_grid *g, const PcgWs &w) {
-  ResPlan p = res_plan(g);
+  // a withheld exchange (failure tests) needs waits that can run out
+  ResPlan p = res_plan(g, g_withhold1.load() ? 0 : res_cluster_ctas());
   const size_t NN = (size_t)(g->nelx + 1) * w.P;
-  if (p && 2 * res_words(g, p) > 10 * NN) p.threads = 0;  // wa, wb, sa, sb, pa
+  if (p && !p.cluster && 2 * res_words(g, p) > 10 * NN) p.threads = 0;  // wa, wb, sa, sb, pa
   return p;
 }
 
 template <int PRE>
 int launch_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const double *f,
                const uint8_t *fixed, double *u, const PcgWs &w, const ResPlan &p,
-               cudaStream_t st, cudaEvent_t *ev) {
+               tpo_solve_result *out, cudaStream_t st, cudaEvent_t *ev) {
   const double fn = std::sqrt(c->f_norm_sq);
-  const size_t words = res_words(g, p), nodes = (size_t)(g->nelx + 1) * (g->nely + 1);
-  k_res_init<<<flat_grid(words, 256, sm_count() * 8), 256, 0, st>>>(
-      reinterpret_cast<double2 *>(w.wa), words, w.ctl, (c->tol * fn) * (c->tol * fn), c->max_iter);
-  TPO_CK_LAUNCH();
+  const size_t nodes = (size_t)(g->nelx + 1) * (g->nely + 1);
   ResArgs a{};
   a.nx = g->nelx;
   a.ny = g->nely;
@@ -910,31 +987,44 @@ int launch_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, con
   a.fixed = fixed;
   a.u = u;
   a.warm = c->warm_start != 0;
-  for (int b = 0; b < 2; ++b)
-    for (int k = 0; k < 2; ++k) a.halo[b][k] = w.wa + 2 * nodes * (2 * b + k);
-  a.sums = w.wa + 8 * nodes;
+  a.tol_sq = (c->tol * fn) * (c->tol * fn);
+  a.max_iter = c->max_iter;
   a.ctl = w.ctl;
-  a.withhold1 = g_withhold1.exchange(0);
+  if (p.cluster) {
+    a.out = out;
+  } else {
+    const size_t words = res_words(g, p);
+    for (int b = 0; b < 2; ++b)
+      for (int k = 0; k < 2; ++k) a.halo[b][k] = w.wa + 2 * nodes * (2 * b + k);
+    a.sums = w.wa + 8 * nodes;
+    a.withhold1 = g_withhold1.exchange(0);
+    k_res_init<<<flat_grid(words, 256, sm_count() * 8), 256, 0, st>>>(
+        reinterpret_cast<double2 *>(w.wa), words, w.ctl);
+    TPO_CK_LAUNCH();
+  }
+  cudaLaunchConfig_t lc;
+  cudaLaunchAttribute at;
+  res_launch_config(p, st, &lc, &at);
   void *args[] = {&a};
-  const void *kern = p.threads <= 512   ? (const void *)k_cgres<PRE, 512>
-                     : p.threads <= 768 ? (const void *)k_cgres<PRE, 768>
-                                        : (const void *)k_cgres<PRE, RES_MAX_THREADS>;
   if (ev) TPO_CK(cudaEventRecord(ev[0], st));
-  TPO_CK(cudaLaunchCooperativeKernel(kern, dim3(p.tx * p.ty), dim3(p.threads), args,
-                                     res_smem(p.BX, p.BY), st));
+  TPO_CK(cudaLaunchKernelExC(&lc, res_kernel<PRE>(p), args));
   TPO_CK_LAUNCH();
   if (ev) TPO_CK(cudaEventRecord(ev[1], st));
+  if (out && !p.cluster) {
+    k_res_result<<<1, 1, 0, st>>>(w.ctl, c->max_iter, out);
+    TPO_CK_LAUNCH();
+  }
   return TPO_OK;
 }
 
-// Blocking form: the whole solve is two launches.
+// Blocking form: the whole solve is one launch (cluster) or two.
 template <int PRE>
 int pcg_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const double *f,
             const uint8_t *fixed, double *u, const PcgWs &w, const ResPlan &p,
             tpo_solve_result *out, cudaStream_t st) {
   cudaEvent_t *ev = nullptr;
   int rc = g_prof_on ? prof_events(1, &ev) : TPO_OK;
-  if (!rc) rc = launch_res<PRE>(g, c, rho, f, fixed, u, w, p, st, ev);
+  if (!rc) rc = launch_res<PRE>(g, c, rho, f, fixed, u, w, p, nullptr, st, ev);
   if (rc) return rc;
   PcgCtl fin;
   TPO_CK(cudaMemcpyAsync(&fin, w.ctl, sizeof(PcgCtl), cudaMemcpyDeviceToHost, st));
@@ -1182,13 +1272,8 @@ int emit_solve_async(const tpo_grid *g, const tpo_solve_cfg *c, const double *rh
   const double tol_sq = (c->tol * fn) * (c->tol * fn);
   if constexpr (!block) {
     if (w.single)
-      if (const ResPlan rp = res_plan_in(g, w)) {
-        const int rc = launch_res<PRE>(g, c, rho, f, fixed, u, w, rp, st, nullptr);
-        if (rc) return rc;
-        k_res_result<<<1, 1, 0, st>>>(w.ctl, c->max_iter, out);
-        TPO_CK_LAUNCH();
-        return TPO_OK;
-      }
+      if (const ResPlan rp = res_plan_in(g, w))
+        return launch_res<PRE>(g, c, rho, f, fixed, u, w, rp, out, st, nullptr);
   }
   const dim3 sg = flat_grid((size_t)nx * P, 256, sm_count() * 16);
   const int64_t l0 = g_launches.load();
