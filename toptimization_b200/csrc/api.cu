@@ -1735,12 +1735,15 @@ int tpo_pcg_solve_async(const tpo_grid *g, const tpo_solve_cfg *c, const double 
 }
 
 // ------------------------------------------------------------------ sensitivity
+static dim3 sens_grid(const tpo_grid *g) {
+  return flat_grid((size_t)g->nelx * g->nely, S_THREADS, sm_count() * 8);
+}
+
 size_t tpo_sensitivity_workspace_bytes(const tpo_grid *g) {
   if (check_grid(g)) return 0;
-  const dim3 gr((g->nely + S_THREADS - 1) / S_THREADS, (g->nelx + SL - 1) / SL, 1);
   Carve cv(nullptr);
   cv.take<SumCtl>(1);
-  cv.take<double>((size_t)gr.x * gr.y);
+  cv.take<double>((size_t)sens_grid(g).x);
   return cv.off;
 }
 
@@ -1758,10 +1761,10 @@ int tpo_sensitivity(const tpo_grid *g, const double *rho_phys, const double *u, 
   if (ws_bytes < tpo_sensitivity_workspace_bytes(g))
     return fail(TPO_ERR_WORKSPACE, "workspace too small");
   cudaStream_t st = static_cast<cudaStream_t>(s);
-  const dim3 gr((g->nely + S_THREADS - 1) / S_THREADS, (g->nelx + SL - 1) / SL, 1);
+  const dim3 gr = sens_grid(g);
   Carve cv(ws);
   SumCtl *ctl = cv.take<SumCtl>(1);
-  double *part = cv.take<double>((size_t)gr.x * gr.y);
+  double *part = cv.take<double>((size_t)gr.x);
   TPO_CK(cudaMemsetAsync(ctl, 0, sizeof(SumCtl), st));
   k_sensitivity<<<gr, S_THREADS, 0, st>>>(g->nelx, g->nely, g->e_min, g->penalty, rho_phys, u, dc,
                                           part, ctl, compliance_out);
@@ -1787,8 +1790,9 @@ int tpo_sensitivity_noalloc(const tpo_grid *g, const double *rho_phys, const dou
   if (!rho_phys || !u || !dc || !compliance_out) return fail(TPO_ERR_ARGS, "NULL pointer argument");
   if (!aligned(u, 16) || !aligned(rho_phys, 8) || !aligned(dc, 8) || !aligned(compliance_out, 8))
     return fail(TPO_ERR_ARGS, "misaligned pointer (u 16 B, doubles 8 B)");
-  const dim3 gr((g->nely + S_THREADS - 1) / S_THREADS, (g->nelx + SL - 1) / SL, 1);
-  const size_t nb = (size_t)gr.x * gr.y;
+  // the documented limit; the launch itself never has more than 8 CTAs per SM
+  const size_t nb = (size_t)((g->nely + 127) / 128) * ((g->nelx + 15) / 16);
+  const dim3 gr = sens_grid(g);
   if (nb > kSensMaxPartials)
     return fail(TPO_ERR_ARGS,
                 "grid %dx%d needs %zu partial sums; the fixed scratch holds %zu "
@@ -1818,16 +1822,16 @@ static int filter_launch(const tpo_grid *g, double rmin, int mode, const double 
   if (!(rmin > 0.0)) return fail(TPO_ERR_ARGS, "rmin must be > 0");
   const int R = (int)std::ceil(rmin);
   if (R > F_MAXR) return fail(TPO_ERR_ARGS, "ceil(rmin) = %d exceeds %d", R, F_MAXR);
-  const int W = 2 * R + 1, TW = FT + 2 * R;
-  const size_t smem = (size_t)(W * W + TW * TW) * sizeof(double);
+  const size_t smem = (size_t)filter_smem_bytes(R);
+  const double den = filter_den(rmin, R);
   const dim3 gr((g->nely + FT - 1) / FT, (g->nelx + FT - 1) / FT, 1);
   cudaStream_t st = static_cast<cudaStream_t>(s);
   if (mode == F_DENSITY) {
     k_filter<F_DENSITY><<<gr, F_THREADS, smem, st>>>(g->nelx, g->nely, rmin, R, x, rho, out, s_out,
-                                                     s32_out, g->e_min, g->penalty);
+                                                     s32_out, g->e_min, g->penalty, den);
   } else {
     k_filter<F_SENS><<<gr, F_THREADS, smem, st>>>(g->nelx, g->nely, rmin, R, x, rho, out, nullptr,
-                                                  nullptr, g->e_min, g->penalty);
+                                                  nullptr, g->e_min, g->penalty, den);
   }
   TPO_CK_LAUNCH();
   return TPO_OK;

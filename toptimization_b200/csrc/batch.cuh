@@ -46,6 +46,7 @@ struct BDesign {
   int period;                  // takes the PCG steps i of a loop body with i % period == 0 (0, 1: all)
   int pad1;
   double e_min, pen, volfrac, move, rmin, tol;  // tol: early stop on change (0: none)
+  double fden;                 // filter: weight sum of a whole box
   double tol_sq, rupd2;        // PCG stop (true residual) and replacement thresholds
   // compact fields, reference numbering
   double *rho, *rho_phys, *dc, *dc_filt, *u;
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(F_THREADS)
   const int loc = blockIdx.x - J.cta0;
   const double *x = which ? D.dc : D.rho;
   double *out = which ? D.dc_filt : D.rho_phys;
-  filter_run<F_DENSITY>(D.nx, D.ny, D.rmin, D.R, x, nullptr, out, nullptr, nullptr, 0.0, 0.0,
+  filter_run<F_DENSITY>(D.nx, D.ny, D.rmin, D.R, x, nullptr, out, nullptr, nullptr, 0.0, 0.0, D.fden,
                         loc % J.gx, loc / J.gx);
 }
 
@@ -250,9 +251,8 @@ __global__ void __launch_bounds__(S_THREADS) kb_sens(const BJob *jobs, int nj, c
   const BJob &J = find_job(jobs, nj);
   const BDesign &D = ds[J.slot];
   if (!D.active || D.phase != PH_POST) return;
-  const int loc = blockIdx.x - J.cta0;
-  sensitivity_run(D.nx, D.ny, D.e_min, D.pen, D.rho_phys, D.u, D.dc, D.spart, D.sc, D.scal,
-                  loc % J.gx, loc / J.gx, J.gx * J.gy, loc);
+  sensitivity_run(D.nx, D.ny, D.e_min, D.pen, D.rho_phys, D.u, D.dc, D.spart, D.sc, D.scal, J.gx,
+                  blockIdx.x - J.cta0);
 }
 
 // OC update (oc_run, design.cuh), one cluster per design, in place. s goes to

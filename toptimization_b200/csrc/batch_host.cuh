@@ -80,8 +80,7 @@ void kind_geom(int kind, int nx, int ny, int P, int Ls, int Lu, int *gx, int *gy
       *L = Lu;
       break;
     default:  // BK_SENS
-      *gx = cdiv(ny, S_THREADS);
-      *gy = cdiv(nx, SL);
+      *gx = flat_ctas((int64_t)nx * ny, S_THREADS);
       break;
   }
 }
@@ -158,11 +157,6 @@ int check_design(const tpo_batch_design *d) {
   return TPO_OK;
 }
 
-int filter_smem_bytes(int R) {
-  const int W = 2 * R + 1, TW = FT + 2 * R;
-  return (W * W + TW * TW) * (int)sizeof(double);
-}
-
 template <int PRE> int batch_set_attrs() {
   constexpr int SMEM = TsGeom<double, M_RESX>::template slot_bytes<kBatchG>() * kBatchNG;
   constexpr int SMEM_D = TsGeom<float, M_DIR>::template slot_bytes<kBatchG>() * kBatchNG;
@@ -176,7 +170,7 @@ template <int PRE> int batch_set_attrs() {
 // rebuild the job tables of every kind from the active slots
 int batch_rebuild(tpo_batch *b, cudaStream_t st) {
   std::vector<BJob> h((size_t)kBK * b->max_designs);
-  int maxR = 1;
+  int fsm = 0;
   unsigned mb = 4;
   for (int k = 0; k < kBK; ++k) {
     int n = 0, cta = 0;
@@ -190,14 +184,14 @@ int batch_rebuild(tpo_batch *b, cudaStream_t st) {
       cta += j.gx * j.gy;
       h[(size_t)k * b->max_designs + n++] = j;
       if (k == 0) {
-        maxR = std::max(maxR, D.R);
+        fsm = std::max(fsm, filter_smem_bytes(D.R));
         mb = std::max(mb, (unsigned)(D.max_cg + D.max_outer + 4));
       }
     }
     b->njobs[k] = n;
     b->nctas[k] = cta;
   }
-  b->filter_smem = filter_smem_bytes(maxR);
+  b->filter_smem = fsm;
   b->max_bodies = mb;
   TPO_CK(cudaMemcpyAsync(b->d_jobs, h.data(), h.size() * sizeof(BJob), cudaMemcpyHostToDevice, st));
   TPO_CK(cudaStreamSynchronize(st));
@@ -546,6 +540,7 @@ int tpo_batch_add(tpo_batch *b, const tpo_batch_design *d, const double *f, cons
   D.volfrac = d->volfrac;
   D.move = d->move;
   D.rmin = d->rmin;
+  D.fden = filter_den(d->rmin, D.R);
   D.tol = d->tol;
   D.tol_sq = d->cg_tol * d->cg_tol * d->f_norm_sq;
   D.rupd2 = d->inner_tol * d->inner_tol;

@@ -193,6 +193,19 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double *part, uint3
                                   (int)(blockIdx.y * gridDim.x + blockIdx.x));
 }
 
+// r^pen for the SIMP law in 3D. (The 2D solves keep pow: with capped or long
+// PCG runs on a 1e9 contrast a change of the last bit of a scale shows.) Whole exponents 0 to 4 (the usual penalties, and
+// their derivatives') are products, at most two roundings (1.5 ulp, pow: 2 ulp)
+// and a few instructions where pow takes about 150 and 800 cycles of latency.
+__device__ __forceinline__ double simp_pow(double r, double pen) {
+  if (pen == 3.0) return r * r * r;
+  if (pen == 2.0) return r * r;
+  if (pen == 1.0) return r;
+  if (pen == 0.0) return 1.0;
+  if (pen == 4.0) return (r * r) * (r * r);
+  return pow(r, pen);
+}
+
 __device__ __forceinline__ bool finite(double x) { return isfinite(x); }
 
 // ---------------------------------------------------------------- co-resident CTAs

@@ -578,6 +578,42 @@ __host__ __device__ inline H8Const h8_const(double lam, double mu) {
                  (4.0 / 3.0) * mu * q, (4.0 / 9.0) * (lam + 4.0 * mu) * q};
 }
 
+// u^T K u of one element (w = 1): the same transform and modal forces, their
+// product with the modal coefficients instead of the way back to the corners.
+// About 140 operations instead of the 600 multiply-adds of the dense form.
+__host__ __device__ inline double h8_energy(const H8Const &k, const double (&v)[8][3]) {
+  double c[8][3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    double t[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[i] = v[i][j];
+#pragma unroll
+    for (int b = 1; b < 8; b <<= 1)
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (!(i & b)) {
+          const double lo = t[i], hi = t[i + b];
+          t[i] = lo + hi;
+          t[i + b] = hi - lo;
+        }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) c[i][j] = t[i];
+  }
+  const double *a = c[1], *b = c[2], *d = c[4], *p = c[3], *q = c[6], *r = c[5];
+  auto sq = [](double x) { return x * x; };
+  const double tr = a[0] + b[1] + d[2];
+  const double shear = sq(a[1] + b[0]) + sq(a[2] + d[0]) + sq(b[2] + d[1]);
+  double e = k.L4 * sq(tr) + k.M8 * (sq(a[0]) + sq(b[1]) + sq(d[2])) + k.M4 * shear;
+  // linear gradients: the pairs' sums, the own squares, and W with its parts
+  const double W = (p[2] + r[1]) + q[0];
+  e += k.A * (sq(p[0] + q[2]) + sq(p[1] + r[2]) + sq(r[0] + q[1]));
+  e += k.M4 * (sq(p[0]) + sq(p[1]) + sq(q[1]) + sq(q[2]) + sq(r[0]) + sq(r[2]));
+  e += k.Cc * (sq(W) + sq(p[2]) + sq(q[0]) + sq(r[1]));
+  e += k.K2 * (sq(c[7][0]) + sq(c[7][1]) + sq(c[7][2]));
+  return e;
+}
+
 __host__ __device__ inline void h8_forces(const H8Const &k, double w, const double (&v)[8][3],
                                           double (&f)[8][3]) {
   double c[8][3];
@@ -1015,7 +1051,7 @@ __global__ void k_hex_scales(int64_t ne, const double *__restrict__ rho, double 
                              double alpha_reg, double *__restrict__ s, double *__restrict__ w) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne;
        e += (int64_t)gridDim.x * blockDim.x) {
-    const double v = e_min + pow(rho[e], pen) * (1.0 - e_min);
+    const double v = e_min + simp_pow(rho[e], pen) * (1.0 - e_min);
     s[e] = v;
     if (w) {
       const double sc = fmax(v, alpha_reg);
@@ -1070,6 +1106,8 @@ __global__ void k_hex_zero_fixed(int64_t nn, const uint8_t *__restrict__ mask, d
 // fem/kernels.py:275-308): uKu_e = u_e^T Ke u_e, dc_e = -p rho^(p-1)(1-e_min) uKu_e,
 // c = sum_e (e_min + rho^p (1 - e_min)) uKu_e.
 // ---------------------------------------------------------------------------
+// STRUCT: Ke has the structured form, the energy comes from its modes.
+template <bool STRUCT>
 __global__ void __launch_bounds__(H3_THREADS)
     k_hex_sensitivity(Hex3 g, double e_min, double pen, const double *__restrict__ rho,
                       const double *__restrict__ u, double *__restrict__ dc, double *part,
@@ -1079,34 +1117,45 @@ __global__ void __launch_bounds__(H3_THREADS)
   double acc[1] = {0.0};
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne;
        e += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t col = e / g.nz;
-    const int ez = (int)(e - col * g.nz);
-    const int ex = (int)(col / g.ny);
-    const int ey = (int)(col - (int64_t)ex * g.ny);
+    const int col = (int)e / g.nz;  // a grid has fewer than 2^30 elements
+    const int ez = (int)e - col * g.nz;
+    const int ex = col / g.ny;
+    const int ey = col - ex * g.ny;
     const int64_t n0 = (int64_t)ex * sx + (int64_t)ey * sy + ez;
-    double ue[24];
-#pragma unroll
-    for (int dx = 0; dx < 2; ++dx)
-#pragma unroll
-      for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-        for (int dz = 0; dz < 2; ++dz) {
-          const int b = h8_corner(dx, dy, dz);
-          const double *src = u + 3 * (n0 + dx * sx + dy * sy + dz);
-#pragma unroll
-          for (int j = 0; j < 3; ++j) ue[3 * b + j] = src[j];
-        }
     double uku = 0.0;
+    if constexpr (STRUCT) {
+      double v[8][3];  // corner bits dx + 2 dy + 4 dz
 #pragma unroll
-    for (int i = 0; i < 24; ++i) {
-      double ku = c_ke3[i * 24] * ue[0];
+      for (int i = 0; i < 8; ++i) {
+        const double *src = u + 3 * (n0 + (i & 1) * sx + ((i >> 1) & 1) * sy + (i >> 2));
 #pragma unroll
-      for (int j = 1; j < 24; ++j) ku = fma(c_ke3[i * 24 + j], ue[j], ku);
-      uku = fma(ue[i], ku, uku);
+        for (int j = 0; j < 3; ++j) v[i][j] = src[j];
+      }
+      uku = h8_energy(c_h8s, v);
+    } else {
+      double ue[24];
+#pragma unroll
+      for (int dx = 0; dx < 2; ++dx)
+#pragma unroll
+        for (int dy = 0; dy < 2; ++dy)
+#pragma unroll
+          for (int dz = 0; dz < 2; ++dz) {
+            const int b = h8_corner(dx, dy, dz);
+            const double *src = u + 3 * (n0 + dx * sx + dy * sy + dz);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) ue[3 * b + j] = src[j];
+          }
+#pragma unroll
+      for (int i = 0; i < 24; ++i) {
+        double ku = c_ke3[i * 24] * ue[0];
+#pragma unroll
+        for (int j = 1; j < 24; ++j) ku = fma(c_ke3[i * 24 + j], ue[j], ku);
+        uku = fma(ue[i], ku, uku);
+      }
     }
     const double r = rho[e];
-    dc[e] = -pen * pow(r, pen - 1.0) * (1.0 - e_min) * uku;
-    acc[0] += (e_min + pow(r, pen) * (1.0 - e_min)) * uku;
+    dc[e] = -pen * simp_pow(r, pen - 1.0) * (1.0 - e_min) * uku;
+    acc[0] += (e_min + simp_pow(r, pen) * (1.0 - e_min)) * uku;
   }
   if (!grid_reduce<1>(acc, part, &ctl->counter)) return;
   if (threadIdx.x == 0) *c_out = acc[0];
@@ -1158,6 +1207,59 @@ __global__ void __launch_bounds__(H3_FLAT)
             den += w;
           }
         }
+      }
+    }
+    out[e] = (MODE == F_SENS) ? num / (rho[e] * den + 1e-20) : num / (den + 1e-20);
+  }
+}
+
+// The same filters by a list of the box's neighbours with positive weights, in
+// the reference's order, a kernel argument the host fills in (rmin up to about
+// 4.2: H3_TAPS neighbours). An element whose box lies inside the grid adds the
+// listed neighbours and divides by the common weight sum; the others test each
+// neighbour. The box walk above visits and tests (2 R + 1)^3 candidates per
+// element for the 19 of rmin = 1.5 (51 us at 128x64x64).
+constexpr int H3_TAPS = 304;
+struct Hex3Taps {
+  int n, reach;          // neighbours; largest |offset| along an axis
+  double den;            // sum of their weights
+  double w[H3_TAPS];
+  int8_t d[H3_TAPS][4];  // dx, dy, dz
+};
+static_assert(sizeof(Hex3Taps) + 64 <= 4096, "kernel arguments");
+
+template <int MODE>
+__global__ void __launch_bounds__(H3_FLAT)
+    k_hex_filter_taps(Hex3 g, const __grid_constant__ Hex3Taps t, const double *__restrict__ x,
+                      const double *__restrict__ rho, double *__restrict__ out) {
+  __shared__ double sw[H3_TAPS];
+  __shared__ int so[H3_TAPS];
+  for (int k = threadIdx.x; k < t.n; k += H3_FLAT) {
+    sw[k] = t.w[k];
+    so[k] = (t.d[k][0] * g.ny + t.d[k][1]) * g.nz + t.d[k][2];
+  }
+  __syncthreads();
+  const int ne = (int)g.elems();
+  for (int e = blockIdx.x * H3_FLAT + threadIdx.x; e < ne; e += gridDim.x * H3_FLAT) {
+    const int col = e / g.nz, ez = e - col * g.nz;
+    const int ex = col / g.ny, ey = col - ex * g.ny;
+    const bool inner = ex >= t.reach && ex + t.reach < g.nx && ey >= t.reach &&
+                       ey + t.reach < g.ny && ez >= t.reach && ez + t.reach < g.nz;
+    double num = 0.0, den = t.den;
+    if (inner) {
+#pragma unroll 4
+      for (int k = 0; k < t.n; ++k) {
+        const int j = e + so[k];
+        num = fma(sw[k], (MODE == F_SENS) ? rho[j] * x[j] : x[j], num);
+      }
+    } else {
+      den = 0.0;
+      for (int k = 0; k < t.n; ++k) {
+        const int jx = ex + t.d[k][0], jy = ey + t.d[k][1], jz = ez + t.d[k][2];
+        if (jx < 0 || jx >= g.nx || jy < 0 || jy >= g.ny || jz < 0 || jz >= g.nz) continue;
+        const int j = e + so[k];
+        num = fma(sw[k], (MODE == F_SENS) ? rho[j] * x[j] : x[j], num);
+        den += sw[k];
       }
     }
     out[e] = (MODE == F_SENS) ? num / (rho[e] * den + 1e-20) : num / (den + 1e-20);

@@ -308,6 +308,30 @@ Sens3Ws carve_sens3(void *base) {
   return w;
 }
 
+// the neighbours with positive weights in the order dx, dy, dz; false if they
+// are more than a launch's list holds
+bool hex_taps(double rmin, int R, Hex3Taps *t) {
+  t->n = 0;
+  t->reach = 0;
+  t->den = 0.0;
+  for (int dx = -R; dx <= R; ++dx)
+    for (int dy = -R; dy <= R; ++dy)
+      for (int dz = -R; dz <= R; ++dz) {
+        const double w = rmin - std::sqrt((double)(dx * dx + dy * dy + dz * dz));
+        if (!(w > 0.0)) continue;
+        if (t->n == H3_TAPS) return false;
+        t->w[t->n] = w;
+        t->d[t->n][0] = (int8_t)dx;
+        t->d[t->n][1] = (int8_t)dy;
+        t->d[t->n][2] = (int8_t)dz;
+        t->d[t->n][3] = 0;
+        t->den += w;
+        t->reach = std::max(t->reach, std::max(std::abs(dx), std::max(std::abs(dy), std::abs(dz))));
+        ++t->n;
+      }
+  return true;
+}
+
 int filter3_launch(const tpo_grid3 *g, double rmin, int mode, const double *x, const double *rho,
                    double *out, tpo_stream s) {
   int rc = check_grid3(g);
@@ -321,6 +345,15 @@ int filter3_launch(const tpo_grid3 *g, double rmin, int mode, const double *x, c
   const Hex3 h = hex_of(g);
   cudaStream_t st = static_cast<cudaStream_t>(s);
   const dim3 gr = hex_flat_grid(h.elems());
+  Hex3Taps taps;
+  if (hex_taps(rmin, R, &taps)) {
+    if (mode == F_SENS)
+      k_hex_filter_taps<F_SENS><<<gr, H3_FLAT, 0, st>>>(h, taps, x, rho, out);
+    else
+      k_hex_filter_taps<F_DENSITY><<<gr, H3_FLAT, 0, st>>>(h, taps, x, nullptr, out);
+    TPO_CK_LAUNCH();
+    return TPO_OK;
+  }
   if (mode == F_SENS)
     k_hex_filter<F_SENS><<<gr, H3_FLAT, smem, st>>>(h, rmin, R, x, rho, out);
   else
@@ -523,8 +556,9 @@ int tpo3_sensitivity(const tpo_grid3 *g, const double *rho_phys, const double *u
   cudaStream_t st = static_cast<cudaStream_t>(s);
   TPO_CK(cudaMemsetAsync(w.ctl, 0, sizeof(SumCtl), st));
   const Hex3 h = hex_of(g);
-  k_hex_sensitivity<<<hex_elem_grid(h), H3_THREADS, 0, st>>>(h, g->e_min, g->penalty, rho_phys,
-                                                            u, dc, w.part, w.ctl, compliance_out);
+  const auto kern = g_h8_structured[dev] ? k_hex_sensitivity<true> : k_hex_sensitivity<false>;
+  kern<<<hex_elem_grid(h), H3_THREADS, 0, st>>>(h, g->e_min, g->penalty, rho_phys, u, dc, w.part,
+                                                w.ctl, compliance_out);
   TPO_CK_LAUNCH();
   return TPO_OK;
 }
