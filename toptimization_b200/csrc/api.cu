@@ -845,72 +845,65 @@ int pcg_mixed(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, cons
 }
 
 // ----------------------------------------------------------------- resident PCG
-// Tiling of the resident solve (k_cgres): the fewest CTAs whose extended tile
-// (tile and halo ring, one node per thread) fits a CTA of T threads. One
-// cluster if 16 CTAs of at most 768 threads hold the grid (its exchange takes
-// about 1 us less, and every further thread adds to the update, the stencil
-// and the sums: at 1024 threads the cooperative form has caught up); otherwise
-// one CTA per SM at most, the smallest T that allows it; none if 1024 threads
-// do not. Measured per iteration, against 13-16 us with one launch each:
-//   cluster:     60x20 1.75 us, 97x41 2.0, 151x49 2.5 (cooperative 2.7, -, 3.0)
-//   cooperative: 160x64 3.1, 200x100 3.7, 400x200 4.9, 460x270 6.3
+// Plan of the resident solve (k_cgres): k_cgstep's strips in groups of 30 rows.
+// One cluster if 16 CTAs hold the groups (its exchange takes about 1 us less
+// than polled words), otherwise one CTA per SM at most; the fewest groups per
+// CTA that allow it; none if 640 threads do not hold them.
+// Measured per iteration, against 13-16 us with one launch each:
+//   cluster:     60x20 2.3 us, 97x41 2.8
+//   cooperative: 151x49 3.9, 200x100 4.5, 400x200 6.8 (17 before), 460x270 8.5 (19)
 struct ResPlan {
-  int BX = 0, BY = 0, tx = 0, ty = 0, threads = 0;
+  int L = 0, groups = 0, units = 0, per_cta = 0;
   bool cluster = false;
-  explicit operator bool() const { return threads > 0; }
-};
-// the tiling with the fewest CTAs for extended tiles of at most T nodes
-int64_t res_tiles(int cx, int cy, int T, ResPlan *p) {
-  int64_t best = INT64_MAX;
-  for (int by = 1; by <= std::min(cy, T / 3 - 2); ++by) {
-    const int bx = std::min(cx, T / (by + 2) - 2);
-    if (bx < 1) break;
-    const int64_t tiles = (int64_t)((cx + bx - 1) / bx) * ((cy + by - 1) / by);
-    if (tiles >= best) continue;
-    best = tiles;
-    p->tx = (cx + bx - 1) / bx;
-    p->ty = (cy + by - 1) / by;
-    p->BX = (cx + p->tx - 1) / p->tx;  // the same tiles, evened out
-    p->BY = (cy + p->ty - 1) / p->ty;
+  int threads() const { return per_cta * res_warps(L) * 32; }
+  int ctas() const { return (units + per_cta - 1) / per_cta; }
+  size_t smem() const {
+    return (size_t)per_cta * res_group_doubles(L, cluster) * sizeof(double);
   }
-  return best;
-}
-ResPlan res_plan(const tpo_grid *g, int cluster_ctas) {
-  const int cx = g->nelx + 1, cy = g->nely + 1;
-  const int most = std::min(sm_count(), RES_MAX_CTAS);
-  const int64_t nodes = (int64_t)cx * cy;
+  explicit operator bool() const { return per_cta > 0; }
+};
+template <int PRE> ResPlan res_plan(const tpo_grid *g, int cluster_ctas) {
   ResPlan p;
-  int64_t tiles = INT64_MAX;
-  if (nodes <= (int64_t)cluster_ctas * RES_CLUSTER_THREADS)
-    for (int T = 128; T <= RES_CLUSTER_THREADS && !p.cluster; T += 32)
-      p.cluster = (tiles = res_tiles(cx, cy, T, &p)) <= cluster_ctas;
-  if (!p.cluster) tiles = INT64_MAX;
-  if (!p.cluster && nodes <= (int64_t)most * RES_MAX_THREADS)
-    for (int T = 256; T <= RES_MAX_THREADS && tiles > most; T += 128)
-      tiles = res_tiles(cx, cy, T, &p);
-  if (tiles <= most)
-    p.threads = std::max(128, ((p.BX + 2) * (p.BY + 2) + 31) / 32 * 32);
+  if ((int64_t)(g->nelx + 1) * (g->nely + 1) > (int64_t)RES_MAX_UNITS * 480) return p;
+  dim3 grid;
+  CgCfg<double, double, PRE>::plan(g->nelx, g->nely, &grid, &p.L);
+  p.groups = (g->nely + 1 + RES_ROWS - 1) / RES_ROWS;
+  p.units = p.groups * (int)grid.y;
+  if (p.units > RES_MAX_UNITS) return p;
+  const int most = std::min(RES_GROUPS, RES_MAX_THREADS / (res_warps(p.L) * 32));
+  for (const bool cluster : {true, false})
+    for (int m = 1; m <= (cluster ? std::min(most, 2) : most) && !p; ++m)
+      if ((p.units + m - 1) / m <= (cluster ? cluster_ctas : sm_count())) {
+        p.per_cta = m;
+        p.cluster = cluster;
+      }
   return p;
 }
 
+// words of one exchange: two doubles per value, [parity][component][node] and
+// [parity][copy][sum][unit]; they lie over the vectors w, s and p of the form
+// with one launch per iteration, which this one keeps in registers
+size_t res_words(const tpo_grid *g, const ResPlan &p) {
+  return 4 * (size_t)(g->nelx + 1) * (g->nely + 1) + 6 * RES_COPIES * (size_t)p.units +
+         6 * RES_LEADERS;
+}
+
 template <int PRE> const void *res_kernel(const ResPlan &p) {
-  if (p.cluster)
-    return p.threads <= 512 ? (const void *)k_cgres<PRE, 512, true>
-                            : (const void *)k_cgres<PRE, RES_CLUSTER_THREADS, true>;
-  return p.threads <= 512   ? (const void *)k_cgres<PRE, 512, false>
-         : p.threads <= 768 ? (const void *)k_cgres<PRE, 768, false>
-                            : (const void *)k_cgres<PRE, RES_MAX_THREADS, false>;
+  if (p.threads() <= 320)
+    return p.cluster ? (const void *)k_cgres<PRE, 320, true> : (const void *)k_cgres<PRE, 320, false>;
+  return p.cluster ? (const void *)k_cgres<PRE, RES_MAX_THREADS, true>
+                   : (const void *)k_cgres<PRE, RES_MAX_THREADS, false>;
 }
 void res_launch_config(const ResPlan &p, cudaStream_t st, cudaLaunchConfig_t *lc,
                        cudaLaunchAttribute *at) {
   *lc = cudaLaunchConfig_t{};
-  lc->gridDim = dim3(p.tx * p.ty);
-  lc->blockDim = dim3(p.threads);
-  lc->dynamicSmemBytes = res_smem(p.BX, p.BY, p.cluster);
+  lc->gridDim = dim3(p.ctas());
+  lc->blockDim = dim3(p.threads());
+  lc->dynamicSmemBytes = p.smem();
   lc->stream = st;
   if (p.cluster) {
     at->id = cudaLaunchAttributeClusterDimension;
-    at->val.clusterDim.x = p.tx * p.ty;
+    at->val.clusterDim.x = p.ctas();
     at->val.clusterDim.y = at->val.clusterDim.z = 1;
   } else {
     at->id = cudaLaunchAttributeCooperative;
@@ -920,51 +913,46 @@ void res_launch_config(const ResPlan &p, cudaStream_t st, cudaLaunchConfig_t *lc
   lc->numAttrs = 1;
 }
 
-// CTAs a cluster of this device can have (16 where a GPC has room, else 8)
-int res_cluster_ctas() {
+// Once per preconditioner: the kernels' shared-memory limits, and the CTAs a
+// cluster of this device can have (16 where a GPC has room for them, else 8).
+template <int PRE> int res_cluster_ctas() {
   static const int n = [] {
-    int ok = 1;
-    auto allow = [&](const void *k, int threads) {
-      ok &= cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
-                cudaSuccess;
-      ResPlan p;
-      p.tx = RES_CLUSTER_CTAS;
-      p.ty = 1;
-      p.BX = threads / 22 - 2;
-      p.BY = 20;
-      p.threads = threads;
-      p.cluster = true;
-      cudaLaunchConfig_t lc;
-      cudaLaunchAttribute at;
-      res_launch_config(p, nullptr, &lc, &at);
-      int c = 0;
-      ok &= cudaOccupancyMaxActiveClusters(&c, k, &lc) == cudaSuccess && c > 0;
-    };
-    allow((const void *)k_cgres<TPO_PRECOND_NONE, 512, true>, 512);
-    allow((const void *)k_cgres<TPO_PRECOND_JACOBI, 512, true>, 512);
-    allow((const void *)k_cgres<TPO_PRECOND_NODAL_BLOCK, 512, true>, 512);
-    allow((const void *)k_cgres<TPO_PRECOND_NONE, RES_CLUSTER_THREADS, true>, RES_CLUSTER_THREADS);
-    allow((const void *)k_cgres<TPO_PRECOND_JACOBI, RES_CLUSTER_THREADS, true>,
-          RES_CLUSTER_THREADS);
-    allow((const void *)k_cgres<TPO_PRECOND_NODAL_BLOCK, RES_CLUSTER_THREADS, true>,
-          RES_CLUSTER_THREADS);
+    bool ok = true;
+    for (const bool cluster : {true, false})
+      for (const int m : {2, 4}) {  // 320 and 640 threads
+        ResPlan p;
+        p.L = kMinStrip;
+        p.groups = 1;
+        p.per_cta = m;
+        p.units = m * RES_CLUSTER_CTAS;
+        p.cluster = cluster;
+        const void *k = res_kernel<PRE>(p);
+        bool good = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         RES_SMEM_MAX) == cudaSuccess;
+        if (cluster) {
+          good = good && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed,
+                                              1) == cudaSuccess;
+          cudaLaunchConfig_t lc;
+          cudaLaunchAttribute at;
+          res_launch_config(p, nullptr, &lc, &at);
+          int c = 0;
+          good = good && cudaOccupancyMaxActiveClusters(&c, k, &lc) == cudaSuccess && c > 0;
+        }
+        ok = ok && good;
+      }
     if (!ok) cudaGetLastError();
     return ok ? RES_CLUSTER_CTAS : kClusterCtas;
   }();
   return n;
 }
 
-// words of one exchange: two doubles per value, [parity][component][node] and
-// [parity][copy][sum][CTA]; they lie over the vectors w, s and p of the form with one
-// launch per iteration, which this one keeps in registers
-size_t res_words(const tpo_grid *g, const ResPlan &p) {
-  return 4 * (size_t)(g->nelx + 1) * (g->nely + 1) + 6 * RES_COPIES * (size_t)p.tx * p.ty;
-}
-ResPlan res_plan_in(const tpo_grid *g, const PcgWs &w) {
+template <int PRE> ResPlan res_plan_in(const tpo_grid *g, const PcgWs &w) {
   // a withheld exchange (failure tests) needs waits that can run out
-  ResPlan p = res_plan(g, g_withhold1.load() ? 0 : res_cluster_ctas());
+  const int cluster = res_cluster_ctas<PRE>();
+  ResPlan p = res_plan<PRE>(g, g_withhold1.load() ? 0 : cluster);
   const size_t NN = (size_t)(g->nelx + 1) * w.P;
-  if (p && !p.cluster && 2 * res_words(g, p) > 10 * NN) p.threads = 0;  // wa, wb, sa, sb, pa
+  if (p && !p.cluster && 2 * res_words(g, p) > 10 * NN) p.per_cta = 0;  // wa, wb, sa, sb, pa
+  if (p && p.smem() > RES_SMEM_MAX) p.per_cta = 0;
   return p;
 }
 
@@ -977,9 +965,10 @@ int launch_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, con
   ResArgs a{};
   a.nx = g->nelx;
   a.ny = g->nely;
-  a.BX = p.BX;
-  a.BY = p.BY;
-  a.tiles_y = p.ty;
+  a.L = p.L;
+  a.groups = p.groups;
+  a.units = p.units;
+  a.per_cta = p.per_cta;
   a.e_min = g->e_min;
   a.pen = g->penalty;
   a.rho = rho;
@@ -997,6 +986,8 @@ int launch_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, con
     for (int b = 0; b < 2; ++b)
       for (int k = 0; k < 2; ++k) a.halo[b][k] = w.wa + 2 * nodes * (2 * b + k);
     a.sums = w.wa + 8 * nodes;
+    a.coef = a.sums + 12 * RES_COPIES * (size_t)p.units;
+    a.leaders = p.units > RES_ALL_UNITS ? RES_LEADERS : 0;
     a.withhold1 = g_withhold1.exchange(0);
     k_res_init<<<flat_grid(words, 256, sm_count() * 8), 256, 0, st>>>(
         reinterpret_cast<double2 *>(w.wa), words, w.ctl);
@@ -1072,7 +1063,7 @@ template <int PRE>
 int pcg_single(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const double *f,
                const uint8_t *fixed, double *u, const PcgWs &w, tpo_solve_result *out,
                cudaStream_t st, double alpha_reg) {
-  if (const ResPlan rp = res_plan_in(g, w))
+  if (const ResPlan rp = res_plan_in<PRE>(g, w))
     return pcg_res<PRE>(g, c, rho, f, fixed, u, w, rp, out, st);
   const int nx = g->nelx, ny = g->nely, P = w.P;
   const double fn = std::sqrt(c->f_norm_sq);
@@ -1272,7 +1263,7 @@ int emit_solve_async(const tpo_grid *g, const tpo_solve_cfg *c, const double *rh
   const double tol_sq = (c->tol * fn) * (c->tol * fn);
   if constexpr (!block) {
     if (w.single)
-      if (const ResPlan rp = res_plan_in(g, w))
+      if (const ResPlan rp = res_plan_in<PRE>(g, w))
         return launch_res<PRE>(g, c, rho, f, fixed, u, w, rp, out, st, nullptr);
   }
   const dim3 sg = flat_grid((size_t)nx * P, 256, sm_count() * 16);

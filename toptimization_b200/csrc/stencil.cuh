@@ -47,37 +47,6 @@ __device__ __forceinline__ V2<T> node_apply(V2<T> LD, V2<T> LM, V2<T> LU, V2<T> 
   return acc;
 }
 
-// The same rows of K for a square-Q4 Ke in FP64, grouped by its six distinct
-// magnitudes (row 0 of Ke: A, B, C, D, E, -B, F, -D): every product is a node
-// value times a sum or difference of element scales that does not change
-// during a solve, 46 multiply-adds instead of 72, and six constants instead of
-// 64, which a loop can keep in registers.
-struct NodeScales {
-  double ll, lh, rl, rh;  // (x-1, y-1), (x-1, y), (x, y-1), (x, y)
-};
-__device__ __forceinline__ double2 node_apply_sym(double2 LD, double2 LM, double2 LU, double2 CD,
-                                                  double2 CM, double2 CU, double2 RD, double2 RM,
-                                                  double2 RU, const NodeScales &s) {
-  const double sr = s.rl + s.rh, sl = s.ll + s.lh, su = s.lh + s.rh, sd = s.ll + s.rl;
-  const double dr = s.rh - s.rl, dl = s.ll - s.lh, du = s.lh - s.rh, dd = s.rl - s.ll;
-  // row x: C (left, right), F (up, down), E (corners), D, B (mixed terms)
-  const double xc = fma(sr, RM.x, sl * LM.x), xf = fma(su, CU.x, sd * CD.x);
-  const double yc = fma(su, CU.y, sd * CD.y), yf = fma(sr, RM.y, sl * LM.y);
-  const double xe = fma(s.ll, LD.x, fma(s.lh, LU.x, fma(s.rl, RD.x, s.rh * RU.x)));
-  const double ye = fma(s.ll, LD.y, fma(s.lh, LU.y, fma(s.rl, RD.y, s.rh * RU.y)));
-  const double xd = fma(dr, RM.y, fma(dl, LM.y, fma(du, CU.y, dd * CD.y)));
-  const double yd = fma(dr, RM.x, fma(dl, LM.x, fma(du, CU.x, dd * CD.x)));
-  const double t = dl + dr;  // ll - lh - rl + rh
-  const double xb = fma(t, CM.y, fma(s.lh, LU.y, fma(-s.ll, LD.y, fma(s.rl, RD.y, -s.rh * RU.y))));
-  const double yb = fma(t, CM.x, fma(s.lh, LU.x, fma(-s.ll, LD.x, fma(s.rl, RD.x, -s.rh * RU.x))));
-  const double S = sl + sr;
-  const double A = c_ke[0], B = c_ke[1], C = c_ke[2], D = c_ke[3], E = c_ke[4], F = c_ke[6];
-  double2 v;
-  v.x = fma(A, S * CM.x, fma(C, xc, fma(F, xf, fma(E, xe, fma(D, xd, B * xb)))));
-  v.y = fma(A, S * CM.y, fma(C, yc, fma(F, yf, fma(E, ye, fma(-D, yd, B * yb)))));
-  return v;
-}
-
 // s * Ke * p_e for one element from its corner values (BL, BR, TR, TL), using
 // Ke = B0^T D B0 + ch (hx hx^T + hy hy^T): the centre strain (ex, ey, g) and
 // the two hourglass amplitudes are formed once, then spread to the corners.
