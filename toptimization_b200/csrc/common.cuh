@@ -193,8 +193,8 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double *part, uint3
                                   (int)(blockIdx.y * gridDim.x + blockIdx.x));
 }
 
-// r^pen for the SIMP law in 3D. (The 2D solves keep pow: with capped or long
-// PCG runs on a 1e9 contrast a change of the last bit of a scale shows.) Whole exponents 0 to 4 (the usual penalties, and
+// r^pen for the SIMP law in 3D and in the 2D compliance. (2D scales and dc keep
+// pow: with PCG runs on a 1e9 contrast a change of their last bit shows.) Whole exponents 0 to 4 (the usual penalties, and
 // their derivatives') are products, at most two roundings (1.5 ulp, pow: 2 ulp)
 // and a few instructions where pow takes about 150 and 800 cycles of latency.
 __device__ __forceinline__ double simp_pow(double r, double pen) {
@@ -221,6 +221,9 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t *p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ void red_release(uint32_t *p, uint32_t v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 // Waits until the counter reaches `target`; about ten seconds at most, after
 // which *err is set and false returned.
 __device__ __forceinline__ bool wait_count(const uint32_t *p, uint32_t target, uint32_t *err) {
@@ -233,15 +236,45 @@ __device__ __forceinline__ bool wait_count(const uint32_t *p, uint32_t target, u
   return false;
 }
 
+// Warp totals of up to eight values with 9 shuffles instead of 5 each: halves,
+// quarters and eighths of the warp first split the values between them.
+// Value k's total ends in lanes 4 k .. 4 k + 3.
+template <int NV> __device__ __forceinline__ double warp_sum_split(const double (&v)[NV], int lane) {
+  static_assert(NV <= 8, "eight values at most");
+  double a[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) a[k] = k < NV ? v[k] : 0.0;
+  const bool h = lane & 16, q = lane & 8, e = lane & 4;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double give = h ? a[k] : a[k + 4], keep = h ? a[k + 4] : a[k];
+    a[k] = keep + __shfl_xor_sync(FULL, give, 16);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const double give = q ? a[k] : a[k + 2], keep = q ? a[k + 2] : a[k];
+    a[k] = keep + __shfl_xor_sync(FULL, give, 8);
+  }
+  const double give = e ? a[0] : a[1], keep = e ? a[1] : a[0];
+  double t = keep + __shfl_xor_sync(FULL, give, 4);
+  t += __shfl_xor_sync(FULL, t, 2);
+  return t + __shfl_xor_sync(FULL, t, 1);
+}
+
 // CTA part of the all-reduce: totals of NV per-thread values over the CTA,
 // value k in lane 0 of warp k (blockDim.x >= 32 NV; sm holds NV * 32 doubles).
 template <int NV, unsigned MAXMASK>
 __device__ __forceinline__ double cta_reduce(const double (&v)[NV], double *sm) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if constexpr (MAXMASK == 0u && NV > 3) {
+    const double t = warp_sum_split<NV>(v, lane);
+    if ((lane & 3) == 0 && lane < 4 * NV) sm[(lane >> 2) * 32 + wid] = t;
+  } else {
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    const double t = ((MAXMASK >> k) & 1u) ? warp_max(v[k]) : warp_sum(v[k]);
-    if (lane == 0) sm[k * 32 + wid] = t;
+    for (int k = 0; k < NV; ++k) {
+      const double t = ((MAXMASK >> k) & 1u) ? warp_max(v[k]) : warp_sum(v[k]);
+      if (lane == 0) sm[k * 32 + wid] = t;
+    }
   }
   __syncthreads();
   double t = 0.0;
@@ -337,13 +370,10 @@ template <int NVMAX> struct GridTeam {
       __syncthreads();
     } else {
       double *pp = part + (size_t)(calls & 1) * NVMAX * n;
-      if (wid < NV && lane == 0) {
-        pp[wid * n + rank()] = t;
-        __threadfence();
-      }
+      if (wid < NV && lane == 0) pp[wid * n + rank()] = t;
       __syncthreads();
-      if (threadIdx.x == 0) {
-        atomicAdd(&bar->arrived, 1u);
+      if (threadIdx.x == 0) {  // the release covers what the barrier ordered before it
+        red_release(&bar->arrived, 1u);
         s.ok = wait_count(&bar->arrived, (uint32_t)(calls + 1) * n, &bar->err) ? 1 : 0;
       }
       __syncthreads();

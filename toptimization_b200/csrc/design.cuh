@@ -17,7 +17,7 @@ namespace tpo {
 // (dx outer, dy inner), skipping w <= 0 and out-of-domain neighbours.
 // ---------------------------------------------------------------------------
 constexpr int FT = 32;           // tile edge (elements)
-constexpr int F_THREADS = 256;   // 32 rows x 8 columns of threads
+constexpr int F_THREADS = 128;
 constexpr int F_MAXR = 16;
 
 enum FilterMode { F_DENSITY = 0, F_SENS = 1 };
@@ -88,15 +88,17 @@ __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
     out[e] = o;
   }
 }
-// Radii up to F_REGR: four rows of a column per thread. For every column dx of
-// the box a thread reads the 2 R + 4 values its rows need once (16-byte shared
-// loads, conflict-free by the pitch) and the R + 1 weights, and adds the chord
-// of positive weights, instead of two shared loads and two tests per
-// neighbour: at rmin = 4 about 14 loads per element instead of 162. An element whose
-// box lies inside the grid takes the weight sum den_in (filter_den). Values and
-// weights are added in the reference's order (dx, then dy). Bound by the FP64
-// multiply-adds (rmin = 4: 45 per element, 5 us at 2048x1024).
+// Radii up to F_REGR: F_ROWS rows of a column per thread. For every column dx
+// of the box a thread reads the 2 R + F_ROWS values its rows need once (16-byte
+// shared loads, conflict-free by the pitch) and the R + 1 weights, and adds the
+// chord of positive weights, instead of two shared loads and two tests per
+// neighbour: at rmin = 4 about 10 loads per element instead of 162. An element
+// whose box lies inside the grid takes the weight sum den_in (filter_den).
+// Values and weights are added in the reference's order (dx, then dy). At rmin = 4
+// on 2048x1024 elements 96 -> 33 us (46 us with the tile staged one load at a time).
 constexpr int F_REGR = 8;
+constexpr int F_ROWS = 8;
+static_assert(F_THREADS / 32 * F_ROWS == FT, "a CTA covers the tile");
 template <int MODE, int R>
 __device__ __forceinline__ void filter_reg(int nx, int ny, double rmin,
                                            const double *__restrict__ x,
@@ -105,7 +107,7 @@ __device__ __forceinline__ void filter_reg(int nx, int ny, double rmin,
                                            float *__restrict__ s32_out, double e_min, double pen,
                                            double den_in, int bx, int by) {
   constexpr int RA = (R + 1) / 2 * 2, TH = FT + 2 * RA, PITCH = TH + 2, TC = FT + 2 * R;
-  constexpr int NV = 2 * RA + 4;
+  constexpr int NV = 2 * RA + F_ROWS;
   static_assert(PITCH % 4 == 2, "16-byte loads of eight lanes fall into distinct banks");
   extern __shared__ __align__(16) double fsm[];
   double *tile = fsm;               // [TC][PITCH], rows from ey0 - RA
@@ -116,29 +118,42 @@ __device__ __forceinline__ void filter_reg(int nx, int ny, double rmin,
     const int dx = k / (R + 1), dy = k % (R + 1);
     wt[k] = rmin - sqrt((double)(dx * dx + dy * dy));
   }
-  for (int k = threadIdx.x; k < TC * TH; k += F_THREADS) {
-    const int tx = k / TH, ty = k - tx * TH;
-    const int gx = ex0 - R + tx, gy = ey0 - RA + ty;
-    double v = 0.0;
-    if (gx >= 0 && gx < nx && gy >= 0 && gy < ny) {
-      const size_t e = (size_t)gx * ny + gy;
-      v = (MODE == F_SENS) ? rho[e] * x[e] : x[e];
-    }
-    tile[tx * PITCH + ty] = v;
-  }
-  __syncthreads();
   if (threadIdx.x <= R) {
     int m = -1;
     for (int dy = 0; dy <= R; ++dy)
-      if (wt[threadIdx.x * (R + 1) + dy] > 0.0) m = dy;
+      if (rmin - sqrt((double)(threadIdx.x * threadIdx.x + dy * dy)) > 0.0) m = dy;
     chord[threadIdx.x] = m;
+  }
+  constexpr int NB = 8;  // loads in flight per thread
+  for (int k0 = threadIdx.x; k0 < TC * TH; k0 += NB * F_THREADS) {
+    double v[NB];
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int k = k0 + i * F_THREADS, tx = k / TH, ty = k - tx * TH;
+      const int gx = ex0 - R + tx, gy = ey0 - RA + ty;
+      v[i] = 0.0;
+      if (k < TC * TH && gx >= 0 && gx < nx && gy >= 0 && gy < ny) {
+        const size_t e = (size_t)gx * ny + gy;
+        v[i] = (MODE == F_SENS) ? rho[e] * x[e] : x[e];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NB; ++i) {
+      const int k = k0 + i * F_THREADS, tx = k / TH, ty = k - tx * TH;
+      if (k < TC * TH) tile[tx * PITCH + ty] = v[i];
+    }
   }
   __syncthreads();
 
-  const int tx = threadIdx.x & 31, r0 = 4 * (threadIdx.x >> 5);
+  const int tx = threadIdx.x & 31, r0 = F_ROWS * (threadIdx.x >> 5);
   const int ex = ex0 + tx, ey = ey0 + r0;
   if (ex >= nx || ey >= ny) return;
-  double num[4] = {0.0, 0.0, 0.0, 0.0};
+  double num[F_ROWS], den[F_ROWS];
+#pragma unroll
+  for (int j = 0; j < F_ROWS; ++j) {
+    num[j] = 0.0;
+    den[j] = den_in;
+  }
 #pragma unroll 1
   for (int dx = -R; dx <= R; ++dx) {
     const int m = chord[abs(dx)];
@@ -157,30 +172,34 @@ __device__ __forceinline__ void filter_reg(int nx, int ny, double rmin,
       if (abs(d) <= m) {
         const double wd = w[abs(d)];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) num[j] = fma(wd, v[RA + j + d], num[j]);
+        for (int j = 0; j < F_ROWS; ++j) num[j] = fma(wd, v[RA + j + d], num[j]);
       }
     }
   }
-  const bool inner = ex >= R && ex + R < nx && ey >= R && ey + 3 + R < ny;
+  const bool inner = ex >= R && ex + R < nx && ey >= R && ey + F_ROWS - 1 + R < ny;
+  if (!inner) {  // the weights inside the grid, in the same order
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const int yj = ey + j;
-    if (yj >= ny) break;
-    double den = den_in;
-    if (!inner) {
-      den = 0.0;
-      for (int dx = max(-R, -ex); dx <= min(R, nx - 1 - ex); ++dx) {
-        const int m = chord[abs(dx)];
-        for (int dy = max(-m, -yj); dy <= min(m, ny - 1 - yj); ++dy)
-          den += wt[abs(dx) * (R + 1) + abs(dy)];
+    for (int j = 0; j < F_ROWS; ++j) den[j] = 0.0;
+    for (int dx = max(-R, -ex); dx <= min(R, nx - 1 - ex); ++dx) {
+      const int m = chord[abs(dx)];
+      for (int dy = -m; dy <= m; ++dy) {
+        const double wd = wt[abs(dx) * (R + 1) + abs(dy)];
+#pragma unroll
+        for (int j = 0; j < F_ROWS; ++j)
+          den[j] += (unsigned)(ey + j + dy) < (unsigned)ny ? wd : 0.0;
       }
     }
+  }
+#pragma unroll
+  for (int j = 0; j < F_ROWS; ++j) {
+    const int yj = ey + j;
+    if (yj >= ny) break;
     const size_t e = (size_t)ex * ny + yj;
     double o;
     if (MODE == F_SENS) {
-      o = num[j] / (rho[e] * den + 1e-20);
+      o = num[j] / (rho[e] * den[j] + 1e-20);
     } else {
-      o = num[j] / (den + 1e-20);
+      o = num[j] / (den[j] + 1e-20);
       if (s_out || s32_out) {
         const double s = e_min + pow(o, pen) * (1.0 - e_min);
         if (s_out) s_out[e] = s;
@@ -276,12 +295,12 @@ __device__ __forceinline__ void sensitivity_run(int nx, int ny, double e_min, do
     const double uku = elem_energy(q[0], q[ny + 1], q[ny + 2], q[1]);
     const double r = rho[e];
     dc[e] = -pen * pow(r, pen - 1.0) * (1.0 - e_min) * uku;
-    acc[0] += (e_min + pow(r, pen) * (1.0 - e_min)) * uku;
+    acc[0] += (e_min + simp_pow(r, pen) * (1.0 - e_min)) * uku;
   }
   if (!grid_reduce<1>(acc, part, &ctl->counter, nb, bid)) return;
   if (threadIdx.x == 0) *c_out = acc[0];
 }
-__global__ void __launch_bounds__(S_THREADS)
+__global__ void __launch_bounds__(S_THREADS, 4)
     k_sensitivity(int nx, int ny, double e_min, double pen, const double *__restrict__ rho,
                   const double *__restrict__ u, double *__restrict__ dc, double *part,
                   SumCtl *ctl, double *c_out) {
@@ -357,10 +376,10 @@ struct OcWalk {
       default: return 0.5 * (mh + hi);
     }
   }
-  __device__ __forceinline__ void walk(const double *sum, int n, double volfrac) {
+  // above: bit j set if the volume at value j exceeds the target
+  __device__ __forceinline__ void walk(unsigned above) {
     if (scan == 1) {
-      int j = 0;
-      while (j < OC_NL && !(sum[j] / n > volfrac)) ++j;
+      const int j = above ? __ffs(above) - 1 : OC_NL;
       k0 = OC_NL * j;
       if (k0 >= OC_MAX_STEPS - 1) {  // never: all 50 midpoints are upper bounds
         last = ldexp(1e9, -OC_MAX_STEPS);
@@ -372,8 +391,8 @@ struct OcWalk {
       return;
     }
     if (scan == 2) {
-      int j = 0;
-      while (j < OC_NL - 1 && !(sum[j] / n > volfrac)) ++j;
+      above &= (1u << (OC_NL - 1)) - 1;
+      const int j = above ? __ffs(above) - 1 : OC_NL - 1;
       steps = k0 + j + 1;
       last = lo = ldexp(1e9, -steps);
       hi = ldexp(1e9, -(steps - 1));
@@ -381,16 +400,30 @@ struct OcWalk {
       scan = 0;
       return;
     }
+    // three levels; the stop tests' divisions do not depend on each other
+    double l[3], h[3], m[3], a = lo, b = hi;
+    bool stop[3];
     int j = 0;
-    for (int level = 0; level < 3 && !done; ++level) {
-      const double m = 0.5 * (lo + hi);
-      last = m;
-      steps += 1;
-      const bool up = sum[j] / n > volfrac;
-      if (up) lo = m; else hi = m;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      m[i] = 0.5 * (a + b);
+      const bool up = (above >> j) & 1u;
+      if (up) a = m[i]; else b = m[i];
       j = 2 * j + (up ? 2 : 1);
-      done = (hi - lo) / (hi + lo + 1e-30) < 1e-4 || steps >= OC_MAX_STEPS;
+      l[i] = a;
+      h[i] = b;
     }
+#pragma unroll
+    for (int i = 0; i < 3; ++i) stop[i] = (h[i] - l[i]) / (h[i] + l[i] + 1e-30) < 1e-4;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (!done) {
+        lo = l[i];
+        hi = h[i];
+        last = m[i];
+        steps += 1;
+        done = stop[i] || steps >= OC_MAX_STEPS;
+      }
   }
 };
 static_assert(OC_NL == 7 && OC_NL * OC_NL == OC_MAX_STEPS - 1, "the scan covers k = 1 .. 49");
@@ -430,13 +463,14 @@ __device__ __forceinline__ void oc_run(Team &team, int n, double volfrac, double
   auto decide = [&](const double *sum) {
     if (threadIdx.x < 32) {
       OcWalk w = sh.w;
-      if (sum) w.walk(sum, n, volfrac);
+      const unsigned above =
+          __ballot_sync(FULL, sum && threadIdx.x < OC_NL && sum[threadIdx.x] / n > volfrac);
+      if (sum) w.walk(above);
       else w.init(dv == nullptr);
-      __syncwarp();
       if (threadIdx.x == 0) sh.w = w;
       if (threadIdx.x < OC_NL) {
         const double l = w.lam(threadIdx.x);
-        sh.lam[threadIdx.x] = dv ? l : 1.0 / sqrt(l);
+        sh.lam[threadIdx.x] = dv ? l : rsqrt(l);
       }
     }
     __syncthreads();
