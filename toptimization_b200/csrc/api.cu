@@ -280,10 +280,8 @@ template <auto KERN> int flat_wave(int nx, int ny) {
   }
   return std::min(update_flat_ctas(nx, ny), sm_count() * occ);
 }
-constexpr int kBlkL = 16;
 dim3 blk_grid(int nx, int ny) {
-  const int warps_y = (ny + 1 + RPW - 1) / RPW;
-  return dim3((warps_y + WPC - 1) / WPC, (nx + 1 + kBlkL - 1) / kBlkL, 1);
+  return dim3((ny + 1 + RPW - 1) / RPW, (nx + 1 + BP_L - 1) / BP_L, 1);
 }
 
 // most CTAs any PCG kernel of this grid can have (sizes the partials buffer)
@@ -613,7 +611,7 @@ int pcg_fp64(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const
   b.part = w.part;
   b.ctl = w.ctl;
   if (block) {
-    k_blockpre<double, double, true, kBlkL><<<blk_grid(nx, ny), ST_THREADS, 0, st>>>(b);
+    k_blockpre<double, double, true><<<blk_grid(nx, ny), BP_THREADS, 0, st>>>(b);
     TPO_CK_LAUNCH();
   } else {
     k_precond_flat<double, double, PRE><<<flat_wave<k_precond_flat<double, double, PRE>>(nx, ny),
@@ -657,7 +655,7 @@ int pcg_fp64(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const
     if (ev) TPO_CK(cudaEventRecord(ev[1], st));
     if (ev) TPO_CK(cudaEventRecord(ev[2], st));
     if (block) {
-      k_blockpre<double, double, false, kBlkL><<<blk_grid(nx, ny), ST_THREADS, 0, st>>>(b);
+      k_blockpre<double, double, false><<<blk_grid(nx, ny), BP_THREADS, 0, st>>>(b);
     } else {
       k_update_flat<double, double, PRE>
           <<<flat_wave<k_update_flat<double, double, PRE>>(nx, ny), UF_THREADS, 0, st>>>(up);
@@ -775,8 +773,8 @@ int pcg_mixed(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, cons
     if (ev) TPO_CK(cudaEventRecord(ev[1], st));
     if (ev) TPO_CK(cudaEventRecord(ev[2], st));
     if (block) {
-      k_blockpre<float, double, false, kBlkL, double>
-          <<<blk_grid(nx, ny), ST_THREADS, 0, st>>>(b);
+      k_blockpre<float, double, false, double>
+          <<<blk_grid(nx, ny), BP_THREADS, 0, st>>>(b);
     } else {
       k_update_flat<float, double, PRE, double>
           <<<flat_wave<k_update_flat<float, double, PRE, double>>(nx, ny), UF_THREADS, 0, st>>>(up);
@@ -798,8 +796,8 @@ int pcg_mixed(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, cons
     StencilCfg<double, double, M_RESX, PRE>::launch(st, rx, nx, ny);
     TPO_CK_LAUNCH();
     if (block) {
-      k_blockpre<float, double, true, kBlkL, double>
-          <<<blk_grid(nx, ny), ST_THREADS, 0, st>>>(b);
+      k_blockpre<float, double, true, double>
+          <<<blk_grid(nx, ny), BP_THREADS, 0, st>>>(b);
       TPO_CK_LAUNCH();
     } else {  // z of the replaced residual (no-op when the replacement did not run)
       k_precond_flat<float, double, PRE><<<flat_wave<k_precond_flat<float, double, PRE>>(nx, ny),
@@ -1309,7 +1307,7 @@ int emit_solve_async(const tpo_grid *g, const tpo_solve_cfg *c, const double *rh
       if (block) {
         BlkArgs bi = b;
         bi.gate = 1;
-        k_blockpre<float, double, true, kBlkL, double><<<blk_grid(nx, ny), ST_THREADS, 0, bs>>>(bi);
+        k_blockpre<float, double, true, double><<<blk_grid(nx, ny), BP_THREADS, 0, bs>>>(bi);
       } else {
         k_precond_gated<float, double, PRE>
             <<<flat_wave<k_precond_gated<float, double, PRE>>(nx, ny), UF_THREADS, 0, bs>>>(
@@ -1320,7 +1318,7 @@ int emit_solve_async(const tpo_grid *g, const tpo_solve_cfg *c, const double *rh
         StencilCfg<float, double, M_DIR, TPO_PRECOND_BLOCK_JACOBI>::launch(bs, d, nx, ny);
         TPO_CK_LAUNCH();
         if (block)
-          k_blockpre<float, double, false, kBlkL, double><<<blk_grid(nx, ny), ST_THREADS, 0, bs>>>(b);
+          k_blockpre<float, double, false, double><<<blk_grid(nx, ny), BP_THREADS, 0, bs>>>(b);
         else
           k_update_flat<float, double, PRE, double>
               <<<flat_wave<k_update_flat<float, double, PRE, double>>(nx, ny), UF_THREADS, 0, bs>>>(up);
@@ -1359,7 +1357,7 @@ int emit_solve_async(const tpo_grid *g, const tpo_solve_cfg *c, const double *rh
       b.w = w.w64; b.mask = w.mask; b.u = w.u; b.ap = w.ap; b.pa = w.pa; b.pb = w.pb;
       b.ra = w.ra; b.rb = w.rb; b.z = w.z; b.part = w.part; b.ctl = w.ctl;
       if (block) {
-        k_blockpre<double, double, true, kBlkL><<<blk_grid(nx, ny), ST_THREADS, 0, st>>>(b);
+        k_blockpre<double, double, true><<<blk_grid(nx, ny), BP_THREADS, 0, st>>>(b);
       } else {
         k_precond_flat<double, double, PRE>
             <<<flat_wave<k_precond_flat<double, double, PRE>>(nx, ny), UF_THREADS, 0, st>>>(
@@ -1380,7 +1378,7 @@ int emit_solve_async(const tpo_grid *g, const tpo_solve_cfg *c, const double *rh
           StencilCfg<double, double, M_DIR, TPO_PRECOND_BLOCK_JACOBI>::launch(bs, d, nx, ny);
           TPO_CK_LAUNCH();
           if (block)
-            k_blockpre<double, double, false, kBlkL><<<blk_grid(nx, ny), ST_THREADS, 0, bs>>>(b);
+            k_blockpre<double, double, false><<<blk_grid(nx, ny), BP_THREADS, 0, bs>>>(b);
           else
             k_update_flat<double, double, PRE>
                 <<<flat_wave<k_update_flat<double, double, PRE>>(nx, ny), UF_THREADS, 0, bs>>>(up);

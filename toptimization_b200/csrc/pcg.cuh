@@ -617,119 +617,169 @@ struct BlkArgs {
   int gate;  // INIT: run only right after a residual evaluation (ctl->since == 0)
 };
 
-template <typename T, typename C, bool INIT, int L, typename X = T>
-__global__ void __launch_bounds__(ST_THREADS) k_blockpre(BlkArgs a) {
+// A CTA takes 30 rows x BP_L columns (the strip of one warp of the earlier
+// form, which marched over its columns one load latency after another: 47 us at
+// 801x395, 5 warps per SM). Here every column of the strip and its two
+// neighbours is loaded at once, two per warp, and the 3 x 3 neighbourhoods come
+// from shared memory: 24 us. The arithmetic, and the order of both sums (a row's
+// columns, the rows, groups of four CTAs, then as the last CTA of 128 threads
+// added them), are the earlier form's: the solves it serves amplify a change of
+// one rounding to 1e-6 of u within 40 iterations.
+constexpr int BP_L = 16;                  // own columns
+constexpr int BP_C = BP_L + 2;            // loaded columns
+constexpr int BP_THREADS = BP_C / 2 * 32;
+constexpr int BP_RED_THREADS = ST_THREADS;
+
+// x / sqrt(count of elements at a node): the count is 1, 2 or 4
+template <typename C> __device__ __forceinline__ C div_root_count(C x, int count) {
+  return count == 4 ? C(0.5) * x : count == 1 ? x : x / C(1.4142135623730950488);
+}
+
+template <typename T, typename C, bool INIT, typename X = T>
+__global__ void __launch_bounds__(BP_THREADS) k_blockpre(BlkArgs a) {
   PcgCtl *ctl = a.ctl;
   if (ctl->status != TPO_SOLVE_RUNNING) return;
   if (INIT && a.gate && ctl->since != 0) return;  // no replacement since the last INIT
+  __shared__ V2<C> st[BP_C][32];       // C^-1/2 r of the loaded nodes
+  __shared__ C sw[BP_C][32];           // weights of elements (c, y)
+  __shared__ double sq[2][BP_L][32];   // terms of the sums
+  __shared__ double red[2][BP_RED_THREADS / 32];
+  __shared__ int s_last;
   const int parity = ctl->it & 1;
-  const C alpha = INIT ? C(0) : C(ctl->alpha);
+  const double al = INIT ? 0.0 : ctl->alpha;
+  const C alpha = C(al);
   const T *r_src = static_cast<const T *>(parity ? a.rb : a.ra);
   T *r_dst = static_cast<T *>(parity ? a.ra : a.rb);
   const T *__restrict__ p = static_cast<const T *>(parity ? a.pa : a.pb);
   const int nx = a.nx, ny = a.ny, P = a.P;
-  const int lane = threadIdx.x & 31;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int y = gw * RPW - 1 + lane;
-  const bool row_ok = (y >= 0) && (y <= ny);
-  const bool own_row = row_ok && lane >= 1 && lane <= RPW;
-  const int x0 = blockIdx.y * L;
-  const int x1 = min(x0 + L, nx + 1);
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int y = (int)blockIdx.x * RPW - 1 + lane;
+  const bool row_ok = y >= 0 && y <= ny, own_row = row_ok && lane >= 1 && lane <= RPW;
+  const int x0 = blockIdx.y * BP_L, x1 = min(x0 + BP_L, nx + 1);
   const T *__restrict__ w = static_cast<const T *>(a.w);
   X *__restrict__ u = static_cast<X *>(a.u);
   const T *__restrict__ ap = static_cast<const T *>(a.ap);
   T *__restrict__ z = static_cast<T *>(a.z);
 
-  C e0d = C(0), e0u = C(0), e1d = C(0), e1u = C(0);
-  const V2<C> zero2 = mk2<C>(C(0), C(0));
-  V2<C> n0d = zero2, n0m = zero2, n0u = zero2, n1d = zero2, n1m = zero2, n1u = zero2;
-  V2<C> n2d = zero2, n2m = zero2, n2u = zero2;
-  V2<C> rn1 = zero2, rn2 = zero2;  // unscaled residual at columns c-1, c
-  unsigned m1 = 0, m2 = 0;
-  double acc[2] = {0.0, 0.0};
-
-  struct Raw {
-    C wd, wu;
-    V2<T> r, ap, p;
-    V2<X> u;
-    unsigned m;
-  };
-  const V2<T> tz = mk2<T>(T(0), T(0));
-  auto fetch = [&](int c, Raw &R) {
-    R.wd = R.wu = C(0);
-    const int ce = c - 1;
-    if (ce >= 0 && ce < nx && row_ok) {
-      const size_t e = pslot(ce, y, P);
-      R.wd = C(w[e - 1]);
-      R.wu = C(w[e]);
+  // ---- both columns' loads, then the residual update and C^-1/2 r
+  V2<T> rv[2], av[2], pv[2];
+  V2<X> uv[2];
+  C wv[2];
+  unsigned m[2];
+  bool in[2], own[2];
+  size_t node[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int c = x0 - 1 + 2 * wid + e;
+    in[e] = row_ok && c >= 0 && c <= nx;
+    own[e] = in[e] && own_row && c >= x0 && c < x1;
+    node[e] = in[e] ? pslot(c, y, P) : 0;
+    wv[e] = C(0);
+    m[e] = 0u;
+    if (in[e]) {
+      if (c < nx) wv[e] = C(w[node[e]]);
+      rv[e] = ld2<T>(r_src, node[e]);
+      if (!INIT) av[e] = ld2<T>(ap, node[e]);
     }
-    R.m = 0;
-    R.r = R.ap = R.p = tz;
-    R.u = mk2<X>(X(0), X(0));
-    if (row_ok && c >= 0 && c <= nx) {
-      const size_t node = pslot(c, y, P);
-      R.m = a.mask[node];
-      R.r = ld2<T>(r_src, node);
+    if (own[e]) {
+      m[e] = a.mask[node[e]];
       if (!INIT) {
-        R.ap = ld2<T>(ap, node);
-        if (own_row && c >= x0 && c < x1) {
-          R.u = ld2<X>(u, node);
-          R.p = ld2<T>(p, node);
-        }
+        uv[e] = ld2<X>(u, node[e]);
+        pv[e] = ld2<T>(p, node[e]);
       }
-    }
-  };
-  Raw nxt;
-  fetch(x0 - 1, nxt);
-  for (int c = x0 - 1; c <= x1; ++c) {
-    const Raw cur = nxt;
-    if (c < x1) fetch(c + 1, nxt);
-    e0d = e1d; e0u = e1u;
-    e1d = cur.wd;
-    e1u = cur.wu;
-    V2<C> rt = zero2, rn = zero2;
-    const unsigned m = cur.m;
-    if (row_ok && c >= 0 && c <= nx) {
-      const size_t node = pslot(c, y, P);
-      rn = cvt2<C, T>(cur.r);
-      if (!INIT) {
-        const V2<T> rs = mk2<T>(T(fmaT(-alpha, C(cur.ap.x), rn.x)),
-                                T(fmaT(-alpha, C(cur.ap.y), rn.y)));
-        rn = cvt2<C, T>(rs);
-        if (own_row && c >= x0 && c < x1) {
-          // the solution accumulates in FP64 in every form
-          const double al = ctl->alpha;
-          st2<X>(u, node, mk2<X>(X(fma(al, (double)cur.p.x, (double)cur.u.x)),
-                                 X(fma(al, (double)cur.p.y, (double)cur.u.y))));
-          st2<T>(r_dst, node, rs);
-        }
-      }
-      const C sq = sqrt(C(node_elem_count(c, y, nx, ny)));
-      rt = mk2<C>(rn.x / sq, rn.y / sq);
-    }
-    n0d = n1d; n0m = n1m; n0u = n1u;
-    n1d = n2d; n1m = n2m; n1u = n2u;
-    rn1 = rn2; rn2 = rn;
-    m1 = m2; m2 = m;
-    n2m = rt;
-    n2d = shfl_up2<C>(rt);
-    n2u = shfl_down2<C>(rt);
-
-    const int xo = c - 1;
-    if (own_row && xo >= x0) {
-      const size_t node = pslot(xo, y, P);
-      V2<C> zz = node_apply<C, true>(n0d, n0m, n0u, n1d, n1m, n1u, n2d, n2m, n2u, e0d, e0u, e1d,
-                                     e1u);
-      const C sq = sqrt(C(node_elem_count(xo, y, nx, ny)));
-      const V2<T> zs = mk2<T>((m1 & FIXED_X) ? T(0) : T(zz.x / sq),
-                              (m1 & FIXED_Y) ? T(0) : T(zz.y / sq));
-      st2<T>(z, node, zs);
-      acc[0] += (double)rn1.x * (double)zs.x + (double)rn1.y * (double)zs.y;
-      acc[1] += (double)rn1.x * rn1.x + (double)rn1.y * rn1.y;
     }
   }
-  if (!grid_reduce<2>(acc, a.part, &ctl->counter)) return;
+  V2<C> rn[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    V2<C> rt = mk2<C>(C(0), C(0));
+    rn[e] = rt;
+    if (in[e]) {
+      rn[e] = cvt2<C, T>(rv[e]);
+      if (!INIT) {
+        const V2<T> rs = mk2<T>(T(fmaT(-alpha, C(av[e].x), rn[e].x)),
+                                T(fmaT(-alpha, C(av[e].y), rn[e].y)));
+        rn[e] = cvt2<C, T>(rs);
+        if (own[e]) {
+          // the solution accumulates in FP64 in every form
+          st2<X>(u, node[e], mk2<X>(X(fma(al, (double)pv[e].x, (double)uv[e].x)),
+                                    X(fma(al, (double)pv[e].y, (double)uv[e].y))));
+          st2<T>(r_dst, node[e], rs);
+        }
+      }
+      const int cnt = node_elem_count(x0 - 1 + 2 * wid + e, y, nx, ny);
+      rt = mk2<C>(div_root_count(rn[e].x, cnt), div_root_count(rn[e].y, cnt));
+    }
+    st[2 * wid + e][lane] = rt;
+    sw[2 * wid + e][lane] = wv[e];
+  }
+  __syncthreads();
+
+  // ---- z at the own nodes
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int j = 2 * wid + e;
+    double q0 = 0.0, q1 = 0.0;
+    if (own[e]) {
+      const V2<C> zz = node_apply<C, true>(
+          st[j - 1][lane - 1], st[j - 1][lane], st[j - 1][lane + 1], st[j][lane - 1], st[j][lane],
+          st[j][lane + 1], st[j + 1][lane - 1], st[j + 1][lane], st[j + 1][lane + 1],
+          sw[j - 1][lane - 1], sw[j - 1][lane], sw[j][lane - 1], sw[j][lane]);
+      const int cnt = node_elem_count(x0 - 1 + j, y, nx, ny);
+      const V2<T> zs = mk2<T>((m[e] & FIXED_X) ? T(0) : T(div_root_count(zz.x, cnt)),
+                              (m[e] & FIXED_Y) ? T(0) : T(div_root_count(zz.y, cnt)));
+      st2<T>(z, node[e], zs);
+      q0 = (double)rn[e].x * (double)zs.x + (double)rn[e].y * (double)zs.y;
+      q1 = (double)rn[e].x * rn[e].x + (double)rn[e].y * rn[e].y;
+    }
+    if (j >= 1 && j <= BP_L) {
+      sq[0][j - 1][lane] = q0;
+      sq[1][j - 1][lane] = q1;
+    }
+  }
+  __syncthreads();
+  const int groups = gridDim.x, units = groups * gridDim.y;
+  if (wid < 2) {
+    double s = 0.0;
+    for (int i = 0; i < x1 - x0; ++i) s += sq[wid][i][lane];
+    s = warp_sum(s);
+    if (lane == 0) a.part[(size_t)wid * units + blockIdx.y * groups + blockIdx.x] = s;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&ctl->counter, 1u) == (unsigned)(units - 1);
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (threadIdx.x < BP_RED_THREADS) {
+    const int rows = (groups + WPC - 1) / WPC, nb = rows * (int)gridDim.y;
+    double t[2] = {0.0, 0.0};
+    for (int i = threadIdx.x; i < nb; i += BP_RED_THREADS) {
+      const int s0 = i / rows, g0 = (i - s0 * rows) * WPC, n = min(WPC, groups - g0);
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const double *q = a.part + (size_t)k * units + s0 * groups + g0;
+        double b = __ldcg(q);
+        for (int g = 1; g < n; ++g) b += __ldcg(q + g);
+        t[k] += b;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      t[k] = warp_sum(t[k]);
+      if (lane == 0) red[k][wid] = t[k];
+    }
+  }
+  __syncthreads();
   if (threadIdx.x != 0) return;
+  double acc[2];
+  for (int k = 0; k < 2; ++k) {
+    acc[k] = red[k][0];
+    for (int i = 1; i < BP_RED_THREADS / 32; ++i) acc[k] += red[k][i];
+  }
+  ctl->counter = 0u;
   if (INIT) {
     // first residual of a solve, or (mixed form) a replaced residual
     if (ctl->cont) {
