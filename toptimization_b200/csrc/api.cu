@@ -226,10 +226,12 @@ template <typename T, typename C, int MODE, int PRE> struct StencilCfg {
 };
 
 // Launch configuration of the one-launch iteration (k_cgstep): a ring of NG
-// staged columns per CTA (3 x 11 KB in FP64: six CTAs fit an SM), a grid of
-// about one full wave.
+// staged columns per CTA (4 x 11 KB in FP64, four or five CTAs per SM by
+// registers and shared memory; a solve of 64 iterations with 3 columns 5.03,
+// 2.07, 2.17 ms, with 4: 5.08, 2.00, 2.04, with 5: 5.14, 1.99, 1.99 at
+// 2048x1024, 1201x701, 900x900), a grid of about one full wave.
 template <typename T, typename C, int PRE> struct CgCfg {
-  static constexpr int NG = 3;
+  static constexpr int NG = 4;
   static constexpr int SMEM = CgGeom<T>::SLOT * NG;
   static int resident() {
     static int occ = -1;
@@ -513,12 +515,13 @@ LaunchBytes launch_bytes(const tpo_grid *g) {
   return lb;
 }
 
-// one-launch iteration: r, w, s, p, x read and written, scales, mask
+// one-launch iteration: r, w, s, p read and written, x every second time,
+// scales, mask
 template <typename T>
 LaunchBytes step_bytes(const tpo_grid *g) {
   const int64_t nn = (int64_t)(g->nelx + 1) * (g->nely + 1), nd = 2 * nn;
   const int64_t ne = (int64_t)g->nelx * g->nely, s = sizeof(T);
-  LaunchBytes lb{0, 0, 10 * nd * s + ne * s + nn};
+  LaunchBytes lb{0, 0, 9 * nd * s + ne * s + nn};
   return lb;
 }
 
@@ -554,6 +557,12 @@ int zero_vectors(const PcgWs &w, size_t NN, cudaStream_t st) {
 
 int unpack_solution(const tpo_grid *g, const PcgWs &w, double *u, cudaStream_t st) {
   const size_t n = (size_t)(g->nelx + 1) * (g->nely + 1);
+  if (w.single) {  // the one-launch form may owe u a step
+    k_cg_unpack<<<flat_grid(n, 256, sm_count() * 16), 256, 0, st>>>(g->nelx, g->nely, w.P, w.ctl,
+                                                                    w.u, w.pa, u);
+    TPO_CK_LAUNCH();
+    return TPO_OK;
+  }
   k_unpack_nodes<<<flat_grid(n, 256, sm_count() * 16), 256, 0, st>>>(g->nelx, g->nely, w.P, w.u,
                                                                       u);
   TPO_CK_LAUNCH();

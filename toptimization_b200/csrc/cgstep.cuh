@@ -23,6 +23,12 @@
 // the fixed mask. r, w and s ping-pong between two buffers (strips read their
 // neighbours' columns); p and x are updated in place by their owner only.
 //
+// The solution is brought up to date every second launch, by both steps: x +=
+// alpha_prev p_prev, then += alpha p. p_prev is read anyway, so x is read and
+// written half as often (355 -> 321 MB a launch at 2048x1024 on average, 84.6 -> 78.3 us)
+// with the same operations in the same order. A step still due when the solve
+// ends is added where the solution is unpacked (cg_due).
+//
 // INIT launch (ctl->first = 1): alpha = beta = 0. It forms u = M^-1 r and
 // w = K u for the first residual, p = u, and gamma, delta, ||r||^2, from which
 // the last CTA sets alpha = gamma / delta.
@@ -66,8 +72,11 @@ template <typename T> struct CgGeom {
 // columns, so refills never wait for a consumer warp's arithmetic
 constexpr int CG_THREADS = (WPC + 1) * 32;
 
+// The register count is left to the compiler (94, four CTAs per SM): held at 72
+// for a fifth CTA the launch took 81 instead of 78 us at 2048x1024, at 64 with
+// spills for a sixth 80.
 template <typename T, typename C, int PRE, int NG>
-__global__ void __launch_bounds__(CG_THREADS) k_cgstep(CgArgs A, int L) {
+__global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
   using Geo = CgGeom<T>;
   constexpr int SLOT = Geo::SLOT;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -80,6 +89,8 @@ __global__ void __launch_bounds__(CG_THREADS) k_cgstep(CgArgs A, int L) {
   const C alpha = init ? C(0) : C(ctl->alpha);
   const C beta = init ? C(0) : C(ctl->beta);
   const int par = ctl->phase & 1;
+  const bool both = !init && !par;  // launches 2, 4, ... after INIT update x
+  const C alpha_prev = both ? C(ctl->alpha_prev) : C(0);
   const T *r_in = static_cast<const T *>(par ? A.rb : A.ra);
   const T *w_in = static_cast<const T *>(par ? A.wb : A.wa);
   const T *s_in = static_cast<const T *>(par ? A.sb : A.sa);
@@ -112,7 +123,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_cgstep(CgArgs A, int L) {
     const bool own = c >= x0 && c < x1;
     const bool elem_ok = c >= 0 && c < nx;
     const unsigned bytes = (node_ok ? 3 * Geo::CNB + Geo::CMB : 0) +
-                           (own ? (init ? 1 : 2) * Geo::CNB : 0) + (elem_ok ? Geo::CEB : 0);
+                           (own ? (both ? 2 : 1) * Geo::CNB : 0) + (elem_ok ? Geo::CEB : 0);
     mbar_arrive_expect_tx(bar, bytes);
     const size_t col = 2 * ((size_t)c * P + Y0 + N_OFF);
     if (node_ok) {
@@ -123,7 +134,7 @@ __global__ void __launch_bounds__(CG_THREADS) k_cgstep(CgArgs A, int L) {
     }
     if (own) {
       bulk_g2s(sb + 3 * Geo::CNB, pv + col, Geo::CNB, bar);
-      if (!init) bulk_g2s(sb + 4 * Geo::CNB, xv + col, Geo::CNB, bar);
+      if (both) bulk_g2s(sb + 4 * Geo::CNB, xv + col, Geo::CNB, bar);
     }
     if (elem_ok) bulk_g2s(sb + Geo::OFF_E, gs + (size_t)c * P + Y0 + EWin<T>::OFF, Geo::CEB, bar);
   };
@@ -208,12 +219,17 @@ __global__ void __launch_bounds__(CG_THREADS) k_cgstep(CgArgs A, int L) {
         st2<T>(r_out, o, r_new);
         st2<T>(s_out, o, s_new);
         if (!init) {
-          const V2<T> p_cur = colP[n_idx], x_cur = colX[n_idx];
+          const V2<T> p_cur = colP[n_idx];
           const V2<C> uo = pre_apply<C>(pa, pb, pd, rv);
           const V2<T> pn = mk2<T>(T(fmaT(beta, C(p_cur.x), uo.x)), T(fmaT(beta, C(p_cur.y), uo.y)));
           st2<T>(pv, o, pn);
-          st2<T>(xv, o, mk2<T>(T(fmaT(alpha, C(pn.x), C(x_cur.x))),
-                               T(fmaT(alpha, C(pn.y), C(x_cur.y)))));
+          if (both) {
+            const V2<T> x0 = colX[n_idx];
+            const V2<T> x1 = mk2<T>(T(fmaT(alpha_prev, C(p_cur.x), C(x0.x))),
+                                    T(fmaT(alpha_prev, C(p_cur.y), C(x0.y))));
+            st2<T>(xv, o, mk2<T>(T(fmaT(alpha, C(pn.x), C(x1.x))),
+                                 T(fmaT(alpha, C(pn.y), C(x1.y)))));
+          }
         } else {
           st2<T>(pv, o, mk2<T>(T(un.x), T(un.y)));  // p_0 = u_0
         }
@@ -283,10 +299,35 @@ __global__ void __launch_bounds__(CG_THREADS) k_cgstep(CgArgs A, int L) {
     ctl->status = TPO_SOLVE_BREAKDOWN;
     return;
   }
+  ctl->alpha_prev = ctl->alpha;
   ctl->alpha = gamma / pap;
   ctl->beta = b;
   ctl->rz = gamma;
   ctl->first = 0;
+}
+
+// a step of x is due: an odd number of launches after INIT (ctl->alpha is theirs)
+__device__ __forceinline__ bool cg_due(const PcgCtl *ctl) {
+  return ctl->phase > 1 && !(ctl->phase & 1);
+}
+// the solution in the caller's numbering, with the step that may be due
+__global__ void k_cg_unpack(int nx, int ny, int P, const PcgCtl *ctl,
+                            const double *__restrict__ x, const double *__restrict__ p,
+                            double *__restrict__ dst) {
+  const bool due = cg_due(ctl);
+  const double alpha = ctl->alpha;
+  const size_t total = (size_t)(nx + 1) * (ny + 1);
+  for (size_t n = blockIdx.x * (size_t)blockDim.x + threadIdx.x; n < total;
+       n += (size_t)gridDim.x * blockDim.x) {
+    const int c = (int)(n / (ny + 1)), y = (int)(n % (ny + 1));
+    const size_t i = pslot(c, y, P);
+    double2 v = ld2<double>(x, i);
+    if (due) {
+      const double2 q = ld2<double>(p, i);
+      v = make_double2(fma(alpha, q.x, v.x), fma(alpha, q.y, v.y));
+    }
+    st2<double>(dst, n, v);
+  }
 }
 
 }  // namespace tpo

@@ -95,6 +95,7 @@ struct PcgCtl {
   double beta;      // coefficient of the next direction update
   double rr;        // latest ||r||^2
   double pap;       // latest p.Ap
+  double alpha_prev;  // step length of the iteration before
   double tol_sq;    // stop when rr < tol_sq
   double rupd2;     // mixed form: replace the residual when rr < rupd2 * rmax2 (0: plain)
   double rmax2;     // mixed form: ||r||^2 at the last FP64 residual evaluation

@@ -862,6 +862,7 @@ __device__ __forceinline__ void ctl_init_run(PcgCtl *ctl, double tol_sq, double 
                                              int max_outer) {
   ctl->rz = 0.0;
   ctl->alpha = 0.0;
+  ctl->alpha_prev = 0.0;
   ctl->beta = 0.0;
   ctl->rr = 0.0;
   ctl->pap = 0.0;
