@@ -194,8 +194,9 @@ __device__ __forceinline__ bool grid_reduce(double (&v)[NV], double *part, uint3
                                   (int)(blockIdx.y * gridDim.x + blockIdx.x));
 }
 
-// r^pen for the SIMP law in 3D and in the 2D compliance. (2D scales and dc keep
-// pow: with PCG runs on a 1e9 contrast a change of their last bit shows.) Whole exponents 0 to 4 (the usual penalties, and
+// r^pen for the 3D sensitivities and the 2D compliance. (The solves' scales and
+// 2D dc keep pow: with PCG runs on a 1e9 contrast a change of their last bit
+// shows.) Whole exponents 0 to 4 (the usual penalties, and
 // their derivatives') are products, at most two roundings (1.5 ulp, pow: 2 ulp)
 // and a few instructions where pow takes about 150 and 800 cycles of latency.
 __device__ __forceinline__ double simp_pow(double r, double pen) {

@@ -1051,7 +1051,7 @@ __global__ void k_hex_scales(int64_t ne, const double *__restrict__ rho, double 
                              double alpha_reg, double *__restrict__ s, double *__restrict__ w) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne;
        e += (int64_t)gridDim.x * blockDim.x) {
-    const double v = e_min + simp_pow(rho[e], pen) * (1.0 - e_min);
+    const double v = e_min + pow(rho[e], pen) * (1.0 - e_min);
     s[e] = v;
     if (w) {
       const double sc = fmax(v, alpha_reg);
