@@ -24,8 +24,9 @@ struct tpo_batch {
   // host mirror
   std::vector<tpo::BDesign> rec;
   std::vector<int> used, h_status;
-  int *h_flag = nullptr;        // pinned: 2 poll slots x 4 ints
-  cudaEvent_t ev[2]{};
+  int *h_flag = nullptr;        // host-polled loop only, made on first use (pinning
+  cudaEvent_t ev[2]{};          // takes 1-3 ms): 2 poll slots x 4 ints and their events
+  int h_end[3]{};               // d_flag as last read by batch_read_status
   cudaStream_t cap = nullptr;   // capture stream (graphs cannot be captured on the legacy stream)
   // launch state
   bool dirty = true;
@@ -299,6 +300,11 @@ int batch_round_launches(tpo_batch *b, cudaStream_t st) {
 
 // PCG loop driven from the host: bodies are enqueued two ahead of the flag reads
 int batch_pcg_host(tpo_batch *b, cudaStream_t st) {
+  if (!b->h_flag)
+    TPO_CK(cudaHostAlloc(reinterpret_cast<void **>(&b->h_flag), 8 * sizeof(int),
+                         cudaHostAllocDefault));
+  for (int i = 0; i < 2; ++i)
+    if (!b->ev[i]) TPO_CK(cudaEventCreateWithFlags(&b->ev[i], cudaEventDisableTiming));
   bool pending[2] = {false, false};
   auto issue = [&](int slot) -> int {
     int rc = batch_body_any(b, st, 0, 0);
@@ -382,15 +388,15 @@ int batch_build_round_graph(tpo_batch *b) {
 int batch_read_status(tpo_batch *b, cudaStream_t st) {
   TPO_CK(cudaMemcpyAsync(b->h_status.data(), b->d_status, 2 * (size_t)b->n_slots * sizeof(int),
                          cudaMemcpyDeviceToHost, st));
-  TPO_CK(cudaMemcpyAsync(b->h_flag + 8, b->d_flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
+  TPO_CK(cudaMemcpyAsync(b->h_end, b->d_flag, 3 * sizeof(int), cudaMemcpyDeviceToHost, st));
   TPO_CK(cudaStreamSynchronize(st));
   for (int s = 0; s < b->n_slots; ++s)
     if (b->used[s] && !b->h_status[2 * s + 1] && b->rec[s].active) {
       b->rec[s].active = 0;  // finished on the device: drop it from the job tables
       b->dirty = true;
     }
-  if (b->h_flag[10]) return fail(TPO_ERR_TIMEOUT, "a TMA pipeline wait ran out of time");
-  if (b->h_flag[9]) return fail(TPO_ERR_TIMEOUT, "batched PCG loop stopped at its body limit");
+  if (b->h_end[2]) return fail(TPO_ERR_TIMEOUT, "a TMA pipeline wait ran out of time");
+  if (b->h_end[1]) return fail(TPO_ERR_TIMEOUT, "batched PCG loop stopped at its body limit");
   return TPO_OK;
 }
 
@@ -465,12 +471,6 @@ int tpo_batch_create(int32_t max_designs, const tpo_batch_cfg *cfg, void *ws, si
     tpo_batch_destroy(b);
     return code;
   };
-  if (cudaHostAlloc(reinterpret_cast<void **>(&b->h_flag), 16 * sizeof(int),
-                    cudaHostAllocDefault) != cudaSuccess)
-    return cleanup(fail(TPO_ERR_CUDA, "pinned flag allocation failed"));
-  for (int i = 0; i < 2; ++i)
-    if (cudaEventCreateWithFlags(&b->ev[i], cudaEventDisableTiming) != cudaSuccess)
-      return cleanup(fail(TPO_ERR_CUDA, "event creation failed"));
   if (cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking) != cudaSuccess)
     return cleanup(fail(TPO_ERR_CUDA, "stream creation failed"));
   if (cudaMemset(ws, 0, tpo_batch_workspace_bytes(max_designs)) != cudaSuccess)
