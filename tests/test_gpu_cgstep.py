@@ -1,0 +1,81 @@
+"""The one-launch FP64 iteration beyond the resident sizes (cgstep.cuh), whose
+solution takes two steps every second launch and the last one where it is
+unpacked: odd and even iteration counts, the count reached by convergence and
+by the limit, against the oracle's PCG.
+
+Few iterations with densities in [0.3, 1]: a few hundred ulp at most on either
+side, 1e-11 of the solution; a step that is lost or taken twice is off by the
+step's own size, far above that.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from oracle import simp64 as O  # noqa: E402
+from toptimization_b200 import _lib  # noqa: E402
+from toptimization_b200.fem.solver import PCGSolver  # noqa: E402
+from toptimization_b200.material import compute_Ke_2d, regularized_inverse  # noqa: E402
+
+TOL = 1e-11
+
+
+def _case(nx, ny):
+    rng = np.random.default_rng(nx + ny)
+    Ke = compute_Ke_2d(1.0, 0.3)
+    inv, alpha = regularized_inverse(Ke)
+    _lib.ensure_stiffness(Ke, inv, alpha)
+    fixed = np.arange(2 * (ny + 1))
+    mesh = O.Mesh2D(nx, ny, Ke, fixed)
+    f = rng.standard_normal(mesh.n_dofs)
+    f[mesh.is_fixed] = 0.0
+    mask = np.zeros(mesh.n_nodes, np.uint8)
+    for d in fixed:
+        mask[d // 2] |= 1 << (d % 2)
+    return mesh, f, mask, rng.uniform(0.3, 1.0, nx * ny), 0.1 * rng.standard_normal(mesh.n_dofs)
+
+
+def _both(s, rho, f, mask, u0, warm):
+    dev = lambda a: torch.from_numpy(a).cuda()  # noqa: E731
+    u, v, res = dev(u0.copy()), dev(u0.copy()), s.result_buffer()
+    info = s.solve(dev(rho), dev(f), dev(mask), u, warm_start=warm)
+    s.solve_async(dev(rho), dev(f), dev(mask), v, res, warm_start=warm)
+    torch.cuda.synchronize()
+    got = PCGSolver.decode(res)
+    assert torch.equal(u, v) and (got.updates, got.status) == (info.updates, info.status)
+    return u.cpu().numpy(), info
+
+
+@pytest.mark.parametrize("pre", ["none", "jacobi", "nodal_block_jacobi"])
+@pytest.mark.parametrize("nx,ny", [(433, 401), (3001, 67)])
+def test_every_count(nx, ny, pre):
+    mesh, f, mask, rho, u0 = _case(nx, ny)
+    scale = O.simp_scale(rho, 1e-9, 3.0)
+    for iters, warm in [(1, False), (2, True), (3, False), (4, False), (7, True)]:
+        start = np.where(mesh.is_fixed, 0.0, u0) if warm else np.zeros(mesh.n_dofs)
+        ref = O.pcg(mesh, scale, f, start, 1e-30, iters, pre)
+        s = PCGSolver(nx, ny, 1e-9, 3.0, float(f @ f), preconditioner=pre, max_iter=iters,
+                      tol=1e-30)
+        got, info = _both(s, rho, f, mask, u0, warm)
+        assert info.updates == iters
+        assert np.linalg.norm(got - ref.u) <= TOL * np.linalg.norm(ref.u)
+
+
+@pytest.mark.parametrize("stop", [5, 6])
+def test_converged_at_either_parity(stop):
+    """The tolerance lies halfway between two residuals of the oracle's run."""
+    nx, ny = 433, 401
+    mesh, f, mask, rho, u0 = _case(nx, ny)
+    scale, zero = O.simp_scale(rho, 1e-9, 3.0), np.zeros(mesh.n_dofs)
+    rr = [O.pcg(mesh, scale, f, zero, 1e-30, k, "jacobi").rr for k in range(1, stop + 1)]
+    assert sorted(rr, reverse=True) == rr  # it falls at every step of this run
+    tol = (rr[-1] * rr[-2]) ** 0.25 / np.linalg.norm(f)
+    ref = O.pcg(mesh, scale, f, zero, tol, 50, "jacobi")
+    assert ref.iters == stop
+    s = PCGSolver(nx, ny, 1e-9, 3.0, float(f @ f), preconditioner="jacobi", max_iter=50, tol=tol)
+    got, info = _both(s, rho, f, mask, u0, False)
+    assert info.converged and info.updates == stop
+    assert np.linalg.norm(got - ref.u) <= TOL * np.linalg.norm(ref.u)
