@@ -149,6 +149,29 @@ int check_grid(const tpo_grid *g) {
 }
 
 // ----------------------------------------------------------------- launch plans
+// Launch a kernel that begins with grid_dep(); `dep`: scheduled while the kernel
+// before it in the stream drains (the host-polled PCG loops; a captured loop keeps
+// ordinary launches). The loops are chains of dependent kernels of 15-80 us, each
+// of which began 1-2 us after the last block of the one before: 3442 -> 3320 us
+// (48 mixed iterations, 2048x1024), 5087 -> 4928 (64 in FP64), 4060 -> 3913 (64,
+// 128x64x64), 1506 -> 1439 (40, 61x31x29, element-block). The error, if any, is
+// cudaGetLastError's.
+template <typename... K, typename... A>
+void launch_dep(bool dep, void (*kern)(K...), dim3 grid, int threads, size_t smem,
+                cudaStream_t st, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = dep ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, static_cast<K>(args)...);
+}
+
 dim3 flat_grid(size_t n, int threads, int cap) {
   size_t b = (n + threads - 1) / threads;
   if (b < 1) b = 1;
@@ -212,11 +235,11 @@ template <typename T, typename C, int MODE, int PRE> struct StencilCfg {
     strips = (nx + 1 + L - 1) / L;
     return Plan{dim3(rows, strips, 1), L};
   }
-  static int launch(cudaStream_t st, const TsArgs &a, int nx, int ny) {
+  static int launch(cudaStream_t st, const TsArgs &a, int nx, int ny, bool dep = false) {
     const Plan pl = plan(nx, ny);
     TsArgs b = a;
     b.withhold1 = g_withhold1.exchange(0);  // 0 unless a failure test armed it
-    k_tstencil<T, C, MODE, PRE, G, NG><<<pl.grid, TS_THREADS, SMEM, st>>>(b, pl.L);
+    launch_dep(dep, k_tstencil<T, C, MODE, PRE, G, NG>, pl.grid, TS_THREADS, SMEM, st, b, pl.L);
     return TPO_OK;
   }
   static int max_ctas(int nx, int ny) {
@@ -255,11 +278,11 @@ template <typename T, typename C, int PRE> struct CgCfg {
     *grid = dim3(rows, strips, 1);
     *L = l;
   }
-  static void launch(cudaStream_t st, const CgArgs &a, int nx, int ny) {
+  static void launch(cudaStream_t st, const CgArgs &a, int nx, int ny, bool dep = false) {
     dim3 grid;
     int L;
     plan(nx, ny, &grid, &L);
-    k_cgstep<T, C, PRE, NG><<<grid, CG_THREADS, SMEM, st>>>(a, L);
+    launch_dep(dep, k_cgstep<T, C, PRE, NG>, grid, CG_THREADS, SMEM, st, a, L);
   }
 };
 
@@ -659,15 +682,15 @@ int pcg_fp64(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const
 
   auto iter = [&](cudaEvent_t *ev) -> int {
     if (ev) TPO_CK(cudaEventRecord(ev[0], st));
-    StencilCfg<double, double, M_DIR, TPO_PRECOND_BLOCK_JACOBI>::launch(st, d, nx, ny);  // reads z
+    StencilCfg<double, double, M_DIR, TPO_PRECOND_BLOCK_JACOBI>::launch(st, d, nx, ny, true);
     TPO_CK_LAUNCH();
     if (ev) TPO_CK(cudaEventRecord(ev[1], st));
     if (ev) TPO_CK(cudaEventRecord(ev[2], st));
     if (block) {
-      k_blockpre<double, double, false><<<blk_grid(nx, ny), BP_THREADS, 0, st>>>(b);
+      launch_dep(true, k_blockpre<double, double, false>, blk_grid(nx, ny), BP_THREADS, 0, st, b);
     } else {
-      k_update_flat<double, double, PRE>
-          <<<flat_wave<k_update_flat<double, double, PRE>>(nx, ny), UF_THREADS, 0, st>>>(up);
+      launch_dep(true, k_update_flat<double, double, PRE>,
+                 flat_wave<k_update_flat<double, double, PRE>>(nx, ny), UF_THREADS, 0, st, up);
     }
     TPO_CK_LAUNCH();
     if (ev) TPO_CK(cudaEventRecord(ev[3], st));
@@ -777,16 +800,17 @@ int pcg_mixed(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, cons
 
   auto iter = [&](cudaEvent_t *ev) -> int {
     if (ev) TPO_CK(cudaEventRecord(ev[0], st));
-    StencilCfg<float, double, M_DIR, TPO_PRECOND_BLOCK_JACOBI>::launch(st, d, nx, ny);  // reads z
+    StencilCfg<float, double, M_DIR, TPO_PRECOND_BLOCK_JACOBI>::launch(st, d, nx, ny, true);
     TPO_CK_LAUNCH();
     if (ev) TPO_CK(cudaEventRecord(ev[1], st));
     if (ev) TPO_CK(cudaEventRecord(ev[2], st));
     if (block) {
-      k_blockpre<float, double, false, double>
-          <<<blk_grid(nx, ny), BP_THREADS, 0, st>>>(b);
+      launch_dep(true, k_blockpre<float, double, false, double>, blk_grid(nx, ny), BP_THREADS, 0,
+                 st, b);
     } else {
-      k_update_flat<float, double, PRE, double>
-          <<<flat_wave<k_update_flat<float, double, PRE, double>>(nx, ny), UF_THREADS, 0, st>>>(up);
+      launch_dep(true, k_update_flat<float, double, PRE, double>,
+                 flat_wave<k_update_flat<float, double, PRE, double>>(nx, ny), UF_THREADS, 0, st,
+                 up);
     }
     TPO_CK_LAUNCH();
     if (ev) TPO_CK(cudaEventRecord(ev[3], st));
@@ -1105,7 +1129,7 @@ int pcg_single(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, con
   TPO_CK_LAUNCH();
   auto iter = [&](cudaEvent_t *ev) -> int {
     if (ev) TPO_CK(cudaEventRecord(ev[0], st));
-    CgCfg<double, double, PRE>::launch(st, ca, nx, ny);
+    CgCfg<double, double, PRE>::launch(st, ca, nx, ny, true);
     TPO_CK_LAUNCH();
     if (ev) TPO_CK(cudaEventRecord(ev[1], st));
     return TPO_OK;

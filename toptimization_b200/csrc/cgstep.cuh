@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
   __shared__ __align__(8) uint64_t empty[NG];  // column consumed by all warps
 
   PcgCtl *ctl = A.ctl;
+  grid_dep();
   if (ctl->status != TPO_SOLVE_RUNNING) return;
   const bool init = ctl->first != 0;
   const C alpha = init ? C(0) : C(ctl->alpha);

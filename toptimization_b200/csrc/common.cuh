@@ -40,6 +40,16 @@ template <> __device__ __forceinline__ float kmat<float, false>(int i) { return 
 template <> __device__ __forceinline__ double kmat<double, true>(int i) { return c_kinv[i]; }
 template <> __device__ __forceinline__ float kmat<float, true>(int i) { return c_kinv_f[i]; }
 
+// Start of a kernel of the PCG loop that may be launched while the one before it
+// still runs (launch_dep): waits for the end of that kernel and its memory, then
+// lets the next one be scheduled as this grid's blocks finish. Every thread comes
+// here before its first access to memory, so a kernel that waited stands for all
+// that came before it. Returns at once after an ordinary launch.
+__device__ __forceinline__ void grid_dep() {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+}
+
 // ---------------------------------------------------------------- vectors
 template <typename T> struct V2T;
 template <> struct V2T<double> { typedef double2 type; };

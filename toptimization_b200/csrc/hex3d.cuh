@@ -180,6 +180,7 @@ struct Hex3Args {
 template <int MODE, int PRE>
 __global__ void __launch_bounds__(H3_THREADS) k_hex_gather(Hex3Args a) {
   PcgCtl *ctl = a.ctl;
+  grid_dep();
   if (MODE != H3_APPLY && ctl->status != TPO_SOLVE_RUNNING) return;
   const Hex3 g = a.g;
   const int64_t total = g.nodes();
@@ -344,6 +345,7 @@ __device__ __forceinline__ void cp_async_wait_all() {
 template <int MODE, int PRE>
 __global__ void __launch_bounds__(HT_THREADS, 3) k_hex_tile(Hex3Args a, int xc) {
   PcgCtl *ctl = a.ctl;
+  grid_dep();
   if (MODE != H3_APPLY && ctl->status != TPO_SOLVE_RUNNING) return;
   extern __shared__ double hs[];
   const Hex3 g = a.g;
@@ -720,6 +722,7 @@ __global__ void __launch_bounds__(HE_THREADS, 2)
   static_assert(MODE != H3_BLOCK, "the element-block preconditioner uses the dense gather");
   static_assert(HE_DEPTH >= 2, "the prologue waits for two staged planes");
   PcgCtl *ctl = a.ctl;
+  grid_dep();
   if (MODE != H3_APPLY && ctl->status != TPO_SOLVE_RUNNING) return;
   extern __shared__ double hs[];
   const Hex3 g = a.g;
@@ -967,6 +970,7 @@ __global__ void __launch_bounds__(H3_FLAT)
                  const double *__restrict__ pa, const double *__restrict__ pb,
                  const double *__restrict__ ap, const double *__restrict__ diag,
                  double *__restrict__ z, double *part, PcgCtl *ctl) {
+  grid_dep();
   if (ctl->status != TPO_SOLVE_RUNNING) return;
   const double alpha = ctl->alpha;
   const double *__restrict__ p = (ctl->it & 1) ? pa : pb;  // written by this iteration's direction
@@ -1000,6 +1004,7 @@ __global__ void __launch_bounds__(H3_FLAT)
                   const double *__restrict__ pa, const double *__restrict__ pb,
                   const double *__restrict__ ap, const double *__restrict__ diag,
                   double *__restrict__ z, double *part, PcgCtl *ctl) {
+  grid_dep();
   if (ctl->status != TPO_SOLVE_RUNNING) return;
   const double alpha = ctl->alpha;
   const double *__restrict__ p = (ctl->it & 1) ? pa : pb;  // written by this iteration's direction

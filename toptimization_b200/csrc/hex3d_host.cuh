@@ -133,13 +133,14 @@ GatherPlan gather_plan(const Hex3 &h) {
 }
 
 template <int MODE, int PRE>
-int launch_gather(const GatherPlan &p, const Hex3Args &a, cudaStream_t st) {
+int launch_gather(const GatherPlan &p, const Hex3Args &a, cudaStream_t st, bool dep = false) {
   if constexpr (MODE != H3_BLOCK) {
     if (p.elem) {
       if (p.esmem > 48 * 1024)
         TPO_CK(cudaFuncSetAttribute(k_hex_elem<MODE, PRE>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.esmem));
-      k_hex_elem<MODE, PRE><<<p.egrid, HE_THREADS, p.esmem, st>>>(a, p.ey, p.ez, p.tzc, p.exc);
+      launch_dep(dep, k_hex_elem<MODE, PRE>, p.egrid, HE_THREADS, p.esmem, st, a, p.ey, p.ez, p.tzc,
+                 p.exc);
       TPO_CK_LAUNCH();
       return TPO_OK;
     }
@@ -148,9 +149,9 @@ int launch_gather(const GatherPlan &p, const Hex3Args &a, cudaStream_t st) {
     if (p.smem > 48 * 1024)
       TPO_CK(cudaFuncSetAttribute(k_hex_tile<MODE, PRE>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
-    k_hex_tile<MODE, PRE><<<p.grid, HT_THREADS, p.smem, st>>>(a, p.xc);
+    launch_dep(dep, k_hex_tile<MODE, PRE>, p.grid, HT_THREADS, p.smem, st, a, p.xc);
   } else {
-    k_hex_gather<MODE, PRE><<<p.grid, H3_THREADS, 0, st>>>(a);
+    launch_dep(dep, k_hex_gather<MODE, PRE>, p.grid, H3_THREADS, 0, st, a);
   }
   TPO_CK_LAUNCH();
   return TPO_OK;
@@ -259,18 +260,18 @@ int pcg3(const tpo_grid3 *g, const tpo_solve_cfg *c, const double *rho, const do
 
   auto iter = [&](cudaEvent_t *ev) -> int {
     if (ev) TPO_CK(cudaEventRecord(ev[0], st));
-    int r = launch_gather<H3_DIR, 0>(gp, d, st);
+    int r = launch_gather<H3_DIR, 0>(gp, d, st, true);
     if (r) return r;
     if (ev) TPO_CK(cudaEventRecord(ev[1], st));
     if (ev) TPO_CK(cudaEventRecord(ev[2], st));
     if (vec)
-      k_hex_update2<PRE><<<fg2, H3_FLAT, 0, st>>>(nd, u, w.r, w.pa, w.pb, w.ap, w.diag, w.z,
-                                                  w.part, w.ctl);
+      launch_dep(true, k_hex_update2<PRE>, fg2, H3_FLAT, 0, st, nd, u, w.r, w.pa, w.pb, w.ap,
+                 w.diag, w.z, w.part, w.ctl);
     else
-      k_hex_update<PRE><<<fg, H3_FLAT, 0, st>>>(nd, u, w.r, w.pa, w.pb, w.ap, w.diag, w.z,
-                                                w.part, w.ctl);
+      launch_dep(true, k_hex_update<PRE>, fg, H3_FLAT, 0, st, nd, u, w.r, w.pa, w.pb, w.ap, w.diag,
+                 w.z, w.part, w.ctl);
     TPO_CK_LAUNCH();
-    if (PRE == TPO_PRECOND_BLOCK_JACOBI && (r = launch_gather<H3_BLOCK, 0>(gp, b, st))) return r;
+    if (PRE == TPO_PRECOND_BLOCK_JACOBI && (r = launch_gather<H3_BLOCK, 0>(gp, b, st, true))) return r;
     if (ev) TPO_CK(cudaEventRecord(ev[3], st));
     return TPO_OK;
   };

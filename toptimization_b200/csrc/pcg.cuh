@@ -371,6 +371,7 @@ __device__ __forceinline__ void tstencil_run(const TsArgs &a, int L, int bx, int
 
 template <typename T, typename C, int MODE, int PRE, int G, int NG>
 __global__ void __launch_bounds__(TS_THREADS) k_tstencil(TsArgs a, int L) {
+  grid_dep();
   tstencil_run<T, C, MODE, PRE, G, NG>(a, L, blockIdx.x, blockIdx.y, gridDim.x * gridDim.y,
                                        blockIdx.y * gridDim.x + blockIdx.x);
 }
@@ -590,6 +591,7 @@ __global__ void __launch_bounds__(UF_THREADS) k_precond_gated(const PcgCtl *ctl,
 
 template <typename T, typename C, int PRE, typename X = T>
 __global__ void __launch_bounds__(UF_THREADS) k_update_flat(UpdArgs a) {
+  grid_dep();
   update_flat_run<T, C, PRE, X>(a, blockIdx.x, gridDim.x, gridDim.x, blockIdx.x);
 }
 
@@ -637,6 +639,7 @@ template <typename C> __device__ __forceinline__ C div_root_count(C x, int count
 
 template <typename T, typename C, bool INIT, typename X = T>
 __global__ void __launch_bounds__(BP_THREADS) k_blockpre(BlkArgs a) {
+  grid_dep();
   PcgCtl *ctl = a.ctl;
   if (ctl->status != TPO_SOLVE_RUNNING) return;
   if (INIT && a.gate && ctl->since != 0) return;  // no replacement since the last INIT
