@@ -73,9 +73,10 @@ enum {
 
 /* PCG recurrence. AUTO: one launch per iteration (Chronopoulos-Gear form,
  * one global reduction) for the plain FP64 solve with a point preconditioner
- * (none, Jacobi, nodal block); two launches otherwise (element-block
+ * (none, Jacobi, nodal block), or one for the whole solve where the grid fits
+ * the chip (about 140,000 nodes; the same bits); two launches otherwise (element-block
  * preconditioner, mixed form). STANDARD: the reference's own recurrence
- * (fem/solver.py:27-159), two launches per iteration. SINGLE: the one-launch
+ * (fem/solver.py:27-159), two launches per iteration. SINGLE: AUTO's first
  * form; TPO_ERR_ARGS for the element-block preconditioner or the mixed form
  * (its s = K p recurrence is not kept accurately in FP32 storage). Both forms
  * give the same iterates in exact arithmetic and use the reference's stop,
@@ -172,7 +173,8 @@ int tpo_pcg_solve(const tpo_grid *g, const tpo_solve_cfg *c,
  * reference's fem/solver.py:107-156): no host synchronisation; the PCG loop
  * runs on the device as a CUDA graph conditional WHILE node (bodies of 16
  * iterations, the stop, breakdown and refinement rules decided by the
- * kernels, a bound on the number of bodies), and the result is written to
+ * kernels, a bound on the number of bodies) or, where the grid fits the chip,
+ * inside one kernel (no graph, no bodies), and the result is written to
  * `out_dev`, DEVICE memory (8-byte aligned), when the solve has finished.
  * Same kernels in the same order as tpo_pcg_solve, so the same results.
  * If `s` is capturing, the solve's nodes are added to that capture (so a
@@ -258,7 +260,7 @@ typedef struct tpo_profile {
   int64_t apply_launches;   /* stiffness kernel of tpo_matvec_* / tpo_apply_stiffness_* */
   double apply_ms;
   int64_t apply_bytes;
-  int64_t step_launches;    /* one-launch PCG iteration kernel (TPO_RECURRENCE_SINGLE) */
+  int64_t step_launches;    /* iterations of the one-launch form (TPO_RECURRENCE_SINGLE) */
   double step_ms;
   int64_t step_bytes;
 } tpo_profile;

@@ -2,9 +2,9 @@
 
 Counterpart of the reference's `src/toptimization/optimizer/oc.py:52-93`,
 which bisects lambda from the host with one kernel launch and one sync per
-step. `tpo_oc_update` runs every step on the GPU (the volume reduction, the
-lo/hi move and the stop test happen in the last CTA of each step), with the
-reference's rules: lambda in [0, 1e9], at most 50 steps, stop when
+step. `tpo_oc_update` runs every step in one launch (a pass over the elements
+sums the volumes of the seven midpoints that the next three steps can reach),
+with the reference's rules: lambda in [0, 1e9], at most 50 steps, stop when
 (hi-lo)/(hi+lo+1e-30) < 1e-4, result and max change from the last midpoint.
 Pointwise over elements, so 2D and 3D (`TpoGrid3`) designs share it.
 """
