@@ -79,3 +79,17 @@ def test_converged_at_either_parity(stop):
     got, info = _both(s, rho, f, mask, u0, False)
     assert info.converged and info.updates == stop
     assert np.linalg.norm(got - ref.u) <= TOL * np.linalg.norm(ref.u)
+
+
+@pytest.mark.parametrize("iters,pre,warm", [(1, "jacobi", True), (2, "nodal_block_jacobi", False),
+                                            (5, "none", False), (6, "nodal_block_jacobi", True)])
+def test_alternating_march(iters, pre, warm):
+    """Vectors beyond the L2: every other launch marches in reverse."""
+    nx, ny = 1301, 803
+    mesh, f, mask, rho, u0 = _case(nx, ny)
+    start = np.where(mesh.is_fixed, 0.0, u0) if warm else np.zeros(mesh.n_dofs)
+    ref = O.pcg(mesh, O.simp_scale(rho, 1e-9, 3.0), f, start, 1e-30, iters, pre)
+    s = PCGSolver(nx, ny, 1e-9, 3.0, float(f @ f), preconditioner=pre, max_iter=iters, tol=1e-30)
+    got, info = _both(s, rho, f, mask, u0, warm)
+    assert info.updates == iters
+    assert np.linalg.norm(got - ref.u) <= TOL * np.linalg.norm(ref.u)

@@ -190,6 +190,17 @@ int sm_count() {
   return n;
 }
 
+int l2_bytes() {
+  static int n = 0;
+  if (n == 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrL2CacheSize, dev) != cudaSuccess || n <= 0)
+      n = 126 << 20;
+  }
+  return n;
+}
+
 // Stencil launch configuration per kernel instantiation: dynamic shared
 // memory (set once), resident CTAs per SM, and the strip length that makes
 // the grid close to one full wave.
@@ -249,25 +260,36 @@ template <typename T, typename C, int MODE, int PRE> struct StencilCfg {
 };
 
 // Launch configuration of the one-launch iteration (k_cgstep): a ring of NG
-// staged columns per CTA (4 x 11 KB in FP64, four or five CTAs per SM by
-// registers and shared memory; a solve of 64 iterations with 3 columns 5.03,
-// 2.07, 2.17 ms, with 4: 5.08, 2.00, 2.04, with 5: 5.14, 1.99, 1.99 at
-// 2048x1024, 1201x701, 900x900), a grid of about one full wave.
+// staged columns per CTA (4 x 11 KB in FP64; registers allow four CTAs per SM; with
+// 3, 4 and 5 columns a solve of 64 iterations takes 4.51, 4.54, 4.55 ms at 2048x1024
+// and 2.06, 2.05, 2.04 at 900x900), a grid of about one full wave.
+//
+// Every other launch marches in reverse (k_cgstep<TURN>) where the vectors and
+// scales do not fit the L2. 64 iterations without it and with it: 4.93, 4.53 ms at
+// 2048x1024; 3.08, 2.88 at 1400x850; 2.39, 2.35 at 1250x750, 129 MB; below the
+// L2's 126 MB there is nothing to meet again and the other form is the faster one
+// (2.02, 2.04 at 1201x701; 1.25, 1.26 at 520x400).
 template <typename T, typename C, int PRE> struct CgCfg {
   static constexpr int NG = 4;
   static constexpr int SMEM = CgGeom<T>::SLOT * NG;
   static int resident() {
     static int occ = -1;
     if (occ < 0) {
-      auto kern = k_cgstep<T, C, PRE, NG>;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-      int o = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, CG_THREADS, SMEM) !=
-              cudaSuccess || o < 1)
-        o = 1;
-      occ = o;
+      int least = 0;
+      for (auto kern : {k_cgstep<T, C, PRE, NG, false>, k_cgstep<T, C, PRE, NG, true>}) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        int o = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, CG_THREADS, SMEM) !=
+                cudaSuccess || o < 1)
+          o = 1;
+        least = least ? std::min(least, o) : o;
+      }
+      occ = least;
     }
     return occ;
+  }
+  static bool turn(int nx, int ny) {  // r, w and s twice, p, x; the scales
+    return (8 * 2 * (int64_t)(nx + 1) + nx) * pad_pitch(ny) * (int64_t)sizeof(T) > l2_bytes();
   }
   static void plan(int nx, int ny, dim3 *grid, int *L) {
     const int rows = (ny + 1 + RPC - 1) / RPC;
@@ -282,7 +304,10 @@ template <typename T, typename C, int PRE> struct CgCfg {
     dim3 grid;
     int L;
     plan(nx, ny, &grid, &L);
-    launch_dep(dep, k_cgstep<T, C, PRE, NG>, grid, CG_THREADS, SMEM, st, a, L);
+    if (turn(nx, ny))
+      launch_dep(dep, k_cgstep<T, C, PRE, NG, true>, grid, CG_THREADS, SMEM, st, a, L);
+    else
+      launch_dep(dep, k_cgstep<T, C, PRE, NG, false>, grid, CG_THREADS, SMEM, st, a, L);
   }
 };
 

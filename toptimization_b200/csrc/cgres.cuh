@@ -15,8 +15,9 @@
 // The halo's r and s are kept redundantly, so that w is all that crosses, at
 // the same moment as the sums.
 //
-// Same bits as k_cgstep. A PCG run on a 1e9 contrast amplifies a change of one
-// rounding, so the arithmetic and the order of every sum are k_cgstep's:
+// Same bits as k_cgstep (without TURN, as at all sizes near this one's). A PCG run
+// on a 1e9 contrast amplifies a change of one rounding, so the arithmetic and the
+// order of every sum are k_cgstep's:
 // * A block is the work of one of its CTAs: a strip of L columns x 120 rows, in
 //   up to four groups of 30 rows (one of its warps each). A group has a warp
 //   here for every two columns of the strip and its two neighbours, lanes 0 and

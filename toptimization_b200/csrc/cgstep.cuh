@@ -29,6 +29,13 @@
 // with the same operations in the same order. A step still due when the solve
 // ends is added where the solution is unpacked (cg_due).
 //
+// TURN: every other launch marches from right to left. It begins with the columns
+// the launch before wrote last, which the L2 still holds where it does not hold all
+// vectors (321 MB a launch at 2048x1024, 126 MB of L2), so part of its reads and of
+// the write-backs of p never reach DRAM: 74 -> 68 us a launch. A node's sum is
+// formed in the same order either way (left element, then right); the three sums
+// over a row's columns run in the direction of the march.
+//
 // INIT launch (ctl->first = 1): alpha = beta = 0. It forms u = M^-1 r and
 // w = K u for the first residual, p = u, and gamma, delta, ||r||^2, from which
 // the last CTA sets alpha = gamma / delta.
@@ -72,25 +79,18 @@ template <typename T> struct CgGeom {
 // columns, so refills never wait for a consumer warp's arithmetic
 constexpr int CG_THREADS = (WPC + 1) * 32;
 
-// The register count is left to the compiler (94, four CTAs per SM): held at 72
-// for a fifth CTA the launch took 81 instead of 78 us at 2048x1024, at 64 with
-// spills for a sixth 80.
-template <typename T, typename C, int PRE, int NG>
-__global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
+// One launch, columns from left to right or (REV: odd phases of TURN) from right to left.
+template <typename T, typename C, int PRE, int NG, bool REV>
+__device__ __forceinline__ void cg_run(const CgArgs &A, int L, unsigned char *smem,
+                                       uint64_t *full, uint64_t *empty) {
   using Geo = CgGeom<T>;
   constexpr int SLOT = Geo::SLOT;
-  extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ __align__(8) uint64_t full[NG];   // column staged (TMA transaction bytes)
-  __shared__ __align__(8) uint64_t empty[NG];  // column consumed by all warps
-
   PcgCtl *ctl = A.ctl;
-  grid_dep();
-  if (ctl->status != TPO_SOLVE_RUNNING) return;
-  const bool init = ctl->first != 0;
+  const int par = REV ? 1 : ctl->phase & 1;
+  const bool init = !REV && ctl->first != 0;
   const C alpha = init ? C(0) : C(ctl->alpha);
   const C beta = init ? C(0) : C(ctl->beta);
-  const int par = ctl->phase & 1;
-  const bool both = !init && !par;  // launches 2, 4, ... after INIT update x
+  const bool both = !REV && !init && !par;  // launches 2, 4, ... after INIT update x
   const C alpha_prev = both ? C(ctl->alpha_prev) : C(0);
   const T *r_in = static_cast<const T *>(par ? A.rb : A.ra);
   const T *w_in = static_cast<const T *>(par ? A.wb : A.wa);
@@ -109,20 +109,23 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
   const bool own_row = lane >= 1 && lane <= RPW && y <= ny;
   const int x0 = blockIdx.y * L;
   const int x1 = min(x0 + L, nx + 1);
-  const int cA = x0 - 2;       // first staged column (element scales only)
-  const int NC = x1 - cA + 1;  // staged columns cA..x1
+  // staged columns x0 - 2 .. x1 or, in reverse, x1 + 1 .. x0 - 1, each with the
+  // scales of the elements beyond it; of the first one those alone
+  const int NC = x1 - x0 + 3;
+  auto col_of = [&](int k) { return REV ? x1 + 1 - k : x0 - 2 + k; };
+  auto ecol_of = [&](int c) { return REV ? c - 1 : c; };
   const int ms = (Y0 + LEAD - 1) & ~15;
 
-  // producer (lane 0 of warp WPC): stage column cA + k into ring slot k % NG,
+  // producer (lane 0 of warp WPC): stage column k of the march into ring slot k % NG,
   // after the column that used the slot before (k - NG) has been released by
   // every consumer warp
   auto issue = [&](int k) {
     unsigned char *sb = smem + (k % NG) * SLOT;
     uint64_t *bar = &full[k % NG];
-    const int c = cA + k;
-    const bool node_ok = c > cA && c >= 0 && c <= nx;
+    const int c = col_of(k), ec = ecol_of(c);
+    const bool node_ok = k > 0 && c >= 0 && c <= nx;
     const bool own = c >= x0 && c < x1;
-    const bool elem_ok = c >= 0 && c < nx;
+    const bool elem_ok = ec >= 0 && ec < nx;
     const unsigned bytes = (node_ok ? 3 * Geo::CNB + Geo::CMB : 0) +
                            (own ? (both ? 2 : 1) * Geo::CNB : 0) + (elem_ok ? Geo::CEB : 0);
     mbar_arrive_expect_tx(bar, bytes);
@@ -137,7 +140,7 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
       bulk_g2s(sb + 3 * Geo::CNB, pv + col, Geo::CNB, bar);
       if (both) bulk_g2s(sb + 4 * Geo::CNB, xv + col, Geo::CNB, bar);
     }
-    if (elem_ok) bulk_g2s(sb + Geo::OFF_E, gs + (size_t)c * P + Y0 + EWin<T>::OFF, Geo::CEB, bar);
+    if (elem_ok) bulk_g2s(sb + Geo::OFF_E, gs + (size_t)ec * P + Y0 + EWin<T>::OFF, Geo::CEB, bar);
   };
   bool ok = true;
   if (threadIdx.x == 0) {
@@ -176,12 +179,15 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
 
   const V2<C> zero2 = mk2<C>(C(0), C(0));
   const V2<T> zt = mk2<T>(T(0), T(0));
-  V2<C> un_prev = zero2, uu_prev = zero2, carry = zero2;
-  C sprev_d = C(0), sprev_u = C(0);  // element column c-1, rows y-1, y
+  V2<C> un_prev = zero2, uu_prev = zero2;
+  // the last element's share of the node column it shares with the next: from
+  // the left one element sum, from the right two terms of the node's
+  V2<C> carry = zero2, carry2 = zero2;
+  C sprev_d = C(0), sprev_u = C(0);  // elements between this column and the last, rows y-1, y
   unsigned m_prev = 0;
 
   for (int k = 0; k < NC; ++k) {
-    const int c = cA + k;
+    const int c = col_of(k);
     if (ok) ok = mbar_wait_bounded(&full[k % NG], (k / NG) & 1, A.err, ERR_TMA_TIMEOUT);
     const unsigned char *sb = smem + (k % NG) * SLOT;
     const V2<T> *colR = reinterpret_cast<const V2<T> *>(sb);
@@ -191,10 +197,10 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
     const V2<T> *colX = reinterpret_cast<const V2<T> *>(sb + 4 * Geo::CNB);
     const T *colE = reinterpret_cast<const T *>(sb + Geo::OFF_E);
     const uint8_t *colM = sb + Geo::OFF_M;
-    const bool node_ok = c > cA && c >= 0 && c <= nx;
-    const bool elem_ok = c >= 0 && c < nx;
-    const C scd = elem_ok ? C(colE[e_idx]) : C(0);      // element (c, y-1)
-    const C scu = elem_ok ? C(colE[e_idx + 1]) : C(0);  // element (c, y)
+    const bool node_ok = (REV ? c <= x1 : c > x0 - 2) && c >= 0 && c <= nx;
+    const bool elem_ok = ecol_of(c) >= 0 && ecol_of(c) < nx;
+    const C scd = elem_ok ? C(colE[e_idx]) : C(0);      // element beyond, row y-1
+    const C scu = elem_ok ? C(colE[e_idx + 1]) : C(0);  // element beyond, row y
 
     // ---- node (c, y): s, r updated; u = M^-1 r of the new residual
     V2<C> un = zero2;
@@ -204,7 +210,10 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
       const V2<C> wv = cvt2<C, T>(colW[n_idx]);
       const V2<C> sv = cvt2<C, T>(colS[n_idx]);
       C pa, pb, pd;
-      node_pre<C, PRE>(m, sprev_d, sprev_u, scd, scu, pa, pb, pd);
+      if (REV)
+        node_pre<C, PRE>(m, scd, scu, sprev_d, sprev_u, pa, pb, pd);
+      else
+        node_pre<C, PRE>(m, sprev_d, sprev_u, scd, scu, pa, pb, pd);
       V2<T> s_new, r_new;
       if (init) {
         s_new = zt;
@@ -240,27 +249,34 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
     }
     const V2<C> uu = shfl_down2<C>(un);  // u at (c, y+1)
 
-    // ---- element (c-1, y): corners (c-1,y) (c,y) (c,y+1) (c-1,y+1)
+    // ---- the element of row y between this column and the last
     V2<C> fbl, fbr, ftr, ftl;
-    elem_forces<C>(sprev_u, un_prev, un, uu, uu_prev, fbl, fbr, ftr, ftl);
-    const V2<C> tl_below = shfl_up2<C>(ftl);  // element (c-1, y-1) -> node (c-1, y)
-    const V2<C> tr_below = shfl_up2<C>(ftr);  // element (c-1, y-1) -> node (c, y)
+    if (REV)
+      elem_forces<C>(sprev_u, un, un_prev, uu_prev, uu, fbl, fbr, ftr, ftl);
+    else
+      elem_forces<C>(sprev_u, un_prev, un, uu, uu_prev, fbl, fbr, ftr, ftl);
+    const V2<C> tl_below = shfl_up2<C>(ftl);  // the element of row y-1 -> its left node, row y
+    const V2<C> tr_below = shfl_up2<C>(ftr);  // and its right one
+    V2<C> left = zero2;
+    if (REV) left = mk2<C>(fbr.x + tr_below.x, fbr.y + tr_below.y);
 
     // release the column to the producer
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[k % NG]);
 
-    // ---- w = K u at node (c-1, y) is complete
-    const int xo = c - 1;
-    if (own_row && xo >= x0) {
-      V2<C> wv = mk2<C>(carry.x + fbl.x + tl_below.x, carry.y + fbl.y + tl_below.y);
+    // ---- w = K u at row y of the last column is complete: left element, then right
+    const int xo = REV ? c + 1 : c - 1;
+    if (own_row && (REV ? xo < x1 : xo >= x0)) {
+      V2<C> wv = REV ? mk2<C>(left.x + carry.x + carry2.x, left.y + carry.y + carry2.y)
+                     : mk2<C>(carry.x + fbl.x + tl_below.x, carry.y + fbl.y + tl_below.y);
       if (m_prev & FIXED_X) wv.x = un_prev.x;  // identity rows at fixed DOFs
       if (m_prev & FIXED_Y) wv.y = un_prev.y;
       const V2<T> wt = mk2<T>(T(wv.x), T(wv.y));
       st2<T>(w_out, slot_of(xo), wt);
       acc[1] += (double)un_prev.x * (double)wt.x + (double)un_prev.y * (double)wt.y;
     }
-    carry = mk2<C>(fbr.x + tr_below.x, fbr.y + tr_below.y);
+    carry = REV ? fbl : mk2<C>(fbr.x + tr_below.x, fbr.y + tr_below.y);
+    if (REV) carry2 = tl_below;
     un_prev = un;
     uu_prev = uu;
     sprev_d = scd;
@@ -305,6 +321,24 @@ __global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
   ctl->beta = b;
   ctl->rz = gamma;
   ctl->first = 0;
+}
+
+// The register count is left to the compiler (up to 94, four CTAs per SM): held at
+// 72 for a fifth CTA a solve takes 4.9 instead of 4.5 ms (64 iterations, 2048x1024).
+template <typename T, typename C, int PRE, int NG, bool TURN>
+__global__ void __launch_bounds__(CG_THREADS, 1) k_cgstep(CgArgs A, int L) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  __shared__ __align__(8) uint64_t full[NG];   // column staged (TMA transaction bytes)
+  __shared__ __align__(8) uint64_t empty[NG];  // column consumed by all warps
+  grid_dep();
+  if (A.ctl->status != TPO_SOLVE_RUNNING) return;
+  if constexpr (TURN) {
+    if (A.ctl->phase & 1) {
+      cg_run<T, C, PRE, NG, true>(A, L, smem, full, empty);
+      return;
+    }
+  }
+  cg_run<T, C, PRE, NG, false>(A, L, smem, full, empty);
 }
 
 // a step of x is due: an odd number of launches after INIT (ctl->alpha is theirs)
