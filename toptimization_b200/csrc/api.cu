@@ -969,43 +969,56 @@ void res_launch_config(const ResPlan &p, cudaStream_t st, cudaLaunchConfig_t *lc
   lc->numAttrs = 1;
 }
 
-// Once per preconditioner: the kernels' shared-memory limits, and the CTAs a
-// cluster of this device can have (16 where a GPC has room for them, else 8).
-template <int PRE> int res_cluster_ctas() {
-  static const int n = [] {
-    bool ok = true;
+// What the current device gives k_cgres. Function attributes and cluster sizes are
+// the device's, so both are found out once for each device of the process.
+struct ResDevice {
+  bool usable = false;   // the shared memory every plan may ask for
+  int cluster_ctas = 0;  // CTAs of a cluster: 16 where a GPC has room for them, else 8 (0: none)
+};
+template <int PRE> ResDevice res_device() {
+  static ResDevice devices[kMaxDevices];
+  static std::once_flag once[kMaxDevices];
+  int dev;
+  if (current_device(&dev)) return ResDevice{};
+  std::call_once(once[dev], [&] {
+    ResDevice d;
+    d.usable = true;
     for (const bool cluster : {true, false})
       for (const int m : {2, 4}) {  // 320 and 640 threads
-        ResPlan p;
-        p.L = kMinStrip;
-        p.groups = 1;
-        p.per_cta = m;
-        p.units = m * RES_CLUSTER_CTAS;
-        p.cluster = cluster;
-        const void *k = res_kernel<PRE>(p);
-        bool good = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         RES_SMEM_MAX) == cudaSuccess;
-        if (cluster) {
-          good = good && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                              1) == cudaSuccess;
-          cudaLaunchConfig_t lc;
-          cudaLaunchAttribute at;
-          res_launch_config(p, nullptr, &lc, &at);
-          int c = 0;
-          good = good && cudaOccupancyMaxActiveClusters(&c, k, &lc) == cudaSuccess && c > 0;
-        }
-        ok = ok && good;
+        const void *k = res_kernel<PRE>(ResPlan{kMinStrip, 1, m, m, cluster});
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM_MAX) !=
+            cudaSuccess)
+          d.usable = false;
+        // a refusal leaves the portable size below
+        if (cluster) cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
       }
-    if (!ok) cudaGetLastError();
-    return ok ? RES_CLUSTER_CTAS : kClusterCtas;
-  }();
-  return n;
+    for (const int ctas : {RES_CLUSTER_CTAS, kClusterCtas}) {
+      bool fits = d.usable;
+      for (const int m : {2, 4}) {
+        const ResPlan p{kMinStrip, 1, m * ctas, m, true};
+        cudaLaunchConfig_t lc;
+        cudaLaunchAttribute at;
+        res_launch_config(p, nullptr, &lc, &at);
+        int c = 0;
+        fits = fits && cudaOccupancyMaxActiveClusters(&c, res_kernel<PRE>(p), &lc) == cudaSuccess &&
+               c > 0;
+      }
+      if (fits) {
+        d.cluster_ctas = ctas;
+        break;
+      }
+    }
+    cudaGetLastError();  // of the attempts above
+    devices[dev] = d;
+  });
+  return devices[dev];
 }
 
 template <int PRE> ResPlan res_plan_in(const tpo_grid *g, const PcgWs &w) {
+  const ResDevice d = res_device<PRE>();
+  if (!d.usable) return ResPlan{};
   // a withheld exchange (failure tests) needs waits that can run out
-  const int cluster = res_cluster_ctas<PRE>();
-  ResPlan p = res_plan<PRE>(g, g_withhold1.load() ? 0 : cluster);
+  ResPlan p = res_plan<PRE>(g, g_withhold1.load() ? 0 : d.cluster_ctas);
   const size_t NN = (size_t)(g->nelx + 1) * w.P;
   if (p && !p.cluster && 2 * res_words(g, p) > 10 * NN) p.per_cta = 0;  // wa, wb, sa, sb, pa
   if (p && p.smem() > RES_SMEM_MAX) p.per_cta = 0;
