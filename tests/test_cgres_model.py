@@ -44,3 +44,25 @@ def test_coefficients_wait_for_every_warp_that_reads_them():
             assert buf[re_ % copies] == re_, "a warp reads the coefficients of a later exchange"
             todo.append((w, r + 1, buf))
     assert any(w == 3 * last and r == 2 * last for w, r, _ in seen)
+
+
+def _element_bytes(fn):
+    """Bytes of one element of the vector access in `fn`: what the memory model
+    moves in one piece."""
+    m = re.search(rf"{fn}\(.*?\.global\.v(\d)\.[bu](\d+)", SRC, re.S)
+    assert int(m.group(1)) * int(m.group(2)) == 128
+    return int(m.group(2)) // 8
+
+
+def test_exchanged_word_is_taken_only_when_all_of_it_is_there():
+    """A double travels as 16 bytes, {low word, epoch, high word, epoch}, whose
+    elements may become visible one by one; the reader takes it when both
+    epochs are the current ones. Whatever mix of an old and a new word it
+    sees, what it takes has to be the new value."""
+    size = min(_element_bytes("ll_store"), _element_bytes("ll_load"))
+    old, new = ("old low", 1, "old high", 1), ("new low", 3, "new high", 3)
+    n = 16 // size
+    for arrived in range(1 << n):
+        word = tuple((new if arrived >> (4 * k // size) & 1 else old)[k] for k in range(4))
+        if word[1] == word[3] == 3:
+            assert (word[0], word[2]) == ("new low", "new high"), "an epoch came before its data"

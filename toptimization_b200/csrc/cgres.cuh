@@ -32,8 +32,9 @@
 // one cluster barrier, and the readers fetch them from their owners.
 // Exchange in a cooperative grid, without barriers: a double travels as one
 // 16-byte store of {low word, epoch, high word, epoch}; the reader polls its
-// word until both epochs are the current exchange's (8-byte accesses are
-// single-copy atomic, so data and epoch arrive together). One store and one
+// word until both epochs are the current exchange's (the store's and the load's
+// two elements are 8-byte accesses, each single-copy atomic, so data and epoch
+// arrive together). One store and one
 // load latency instead of fence + arrive + poll + read. Two buffers by parity
 // of the epoch suffice: a CTA publishes exchange e + 2 only after it has all
 // sums of e + 1, which each CTA publishes after it has read all it needs of e.
@@ -87,20 +88,21 @@ struct ResArgs {
   int withhold1;            // failure tests: e + 1 leaves exchange e (0-based) unpublished
 };
 
+// two 8-byte elements, each half of v under the epoch
 __device__ __forceinline__ void ll_store(double *p, size_t i, double v, uint32_t epoch) {
-  const uint64_t x = (uint64_t)__double_as_longlong(v);
-  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(p + 2 * i),
-               "r"((uint32_t)x), "r"(epoch), "r"((uint32_t)(x >> 32))
+  const uint64_t x = (uint64_t)__double_as_longlong(v), e = (uint64_t)epoch << 32;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p + 2 * i),
+               "l"(e | (uint32_t)x), "l"(e | x >> 32)
                : "memory");
 }
 __device__ __forceinline__ bool ll_load(const double *p, size_t i, uint32_t epoch, double &v) {
-  uint32_t a, b, c, d;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(a), "=r"(b), "=r"(c), "=r"(d)
+  uint64_t a, b;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
+               : "=l"(a), "=l"(b)
                : "l"(p + 2 * i)
                : "memory");
-  v = __longlong_as_double((long long)(((uint64_t)c << 32) | a));
-  return b == epoch && d == epoch;
+  v = __longlong_as_double((long long)(b << 32 | (uint32_t)a));
+  return a >> 32 == epoch && b >> 32 == epoch;
 }
 
 // zero the exchange words and the error word
