@@ -327,9 +327,10 @@ __global__ void __launch_bounds__(S_THREADS, 4)
 //   seven midpoints the next three steps can visit, and walks it.
 // The midpoints, their order, the stop test and the step count are those of
 // the one-at-a-time bisection. About 7 passes instead of 50.
-// With dv = 1 the candidate is rho sqrt(-dc / lambda) (lambda + 1e-20 rounds to
-// lambda: it is never below 1e9 / 2^50), so a pass needs s = rho sqrt(-dc) once
-// and then a multiplication, two comparisons and an addition per lambda. s stays
+// With dv = 1 the candidate is rho sqrt(-dc / (lambda + 1e-20)), so a pass needs
+// s = rho sqrt(-dc) once and then a multiplication by 1 / sqrt(lambda + 1e-20),
+// two comparisons and an addition per lambda. (1e-20 is not lost beside lambda:
+// from 1e9 / 2^43 down, the 43rd midpoint, it is part of the sum.) s stays
 // in registers (up to OC_EPT elements per thread) or in `sbuf` (n doubles).
 // The density, its mean and the largest change come from the formula itself.
 // ---------------------------------------------------------------------------
@@ -431,7 +432,7 @@ static_assert(OC_NL == 7 && OC_NL * OC_NL == OC_MAX_STEPS - 1, "the scan covers 
 // What warp 0 decides between two passes, for the whole CTA.
 struct OcShared {
   OcWalk w;
-  double lam[OC_NL];  // with dv: lambda; else 1 / sqrt(lambda)
+  double lam[OC_NL];  // with dv: lambda; else 1 / sqrt(lambda + 1e-20)
 };
 
 // The update of one design by a team of co-resident CTAs of OC_THREADS
@@ -470,7 +471,7 @@ __device__ __forceinline__ void oc_run(Team &team, int n, double volfrac, double
       if (threadIdx.x == 0) sh.w = w;
       if (threadIdx.x < OC_NL) {
         const double l = w.lam(threadIdx.x);
-        sh.lam[threadIdx.x] = dv ? l : rsqrt(l);
+        sh.lam[threadIdx.x] = dv ? l : rsqrt(l + 1e-20);
       }
     }
     __syncthreads();
