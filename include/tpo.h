@@ -131,6 +131,12 @@ const char *tpo_last_error_string(void);
  * TPO_SOLVE_TIMEOUT (tpo_pcg_solve_async). The device stays usable. */
 int tpo_test_withhold_stage(int32_t group);
 
+/* Tests only; no counterpart in the reference. The next solve of the calling
+ * thread that the one-launch recurrence serves runs in this form whatever its
+ * size: 1 a launch per iteration, 2 (where the grid fits the chip) one
+ * cooperative launch. The forms give the same bits (below the L2's size). */
+int tpo_test_solve_form(int32_t form);
+
 /* Element stiffness (8x8 Q4, row-major), its regularised inverse and the
  * regulariser (reference fem/fields.py:133-143), copied to constant memory of
  * the CURRENT device. Must be called once per device before any kernel. */

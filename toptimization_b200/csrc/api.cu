@@ -14,6 +14,7 @@
 #include <vector>
 #include <algorithm>
 #include <atomic>
+#include <utility>
 
 #include "common.cuh"
 #include "design.cuh"
@@ -206,6 +207,9 @@ int l2_bytes() {
 // the grid close to one full wave.
 // failure tests (tpo_test_withhold_stage): group + 1 for the next stencil launch
 std::atomic<int> g_withhold1{0};
+// tests (tpo_test_solve_form): form of this thread's next solve, 0 by its size
+enum SolveForm { FORM_BY_SIZE = 0, FORM_STEPS = 1, FORM_COOPERATIVE = 2 };
+thread_local int t_form = FORM_BY_SIZE;
 
 #ifndef TPO_MIN_STRIP
 #define TPO_MIN_STRIP 8
@@ -1016,9 +1020,11 @@ template <int PRE> ResDevice res_device() {
 
 template <int PRE> ResPlan res_plan_in(const tpo_grid *g, const PcgWs &w) {
   const ResDevice d = res_device<PRE>();
-  if (!d.usable) return ResPlan{};
+  const int form = std::exchange(t_form, (int)FORM_BY_SIZE);
+  if (!d.usable || form == FORM_STEPS) return ResPlan{};
   // a withheld exchange (failure tests) needs waits that can run out
-  ResPlan p = res_plan<PRE>(g, g_withhold1.load() ? 0 : d.cluster_ctas);
+  const bool coop = form == FORM_COOPERATIVE || g_withhold1.load();
+  ResPlan p = res_plan<PRE>(g, coop ? 0 : d.cluster_ctas);
   const size_t NN = (size_t)(g->nelx + 1) * w.P;
   if (p && !p.cluster && 2 * res_words(g, p) > 10 * NN) p.per_cta = 0;  // wa, wb, sa, sb, pa
   if (p && p.smem() > RES_SMEM_MAX) p.per_cta = 0;
@@ -1545,6 +1551,12 @@ static int apply_impl(const tpo_grid *g, const T *elem, bool from_density, const
 extern "C" {
 
 int tpo_version(void) { return 1; }
+
+int tpo_test_solve_form(int32_t form) {
+  if (form < FORM_BY_SIZE || form > FORM_COOPERATIVE) return fail(TPO_ERR_ARGS, "unknown form %d", form);
+  t_form = form;
+  return TPO_OK;
+}
 
 int tpo_test_withhold_stage(int32_t group) {
   if (group < 0) return fail(TPO_ERR_ARGS, "group must be >= 0");

@@ -416,9 +416,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_cgres(ResArgs A) {
       for (int e = 0; e < 2; ++e) {
         double q0 = 0.0, q1 = 0.0, q2 = 0.0;
         if (own[e]) {
-          q0 = r[e].x * u[e].x + r[e].y * u[e].y;
-          q1 = u[e].x * w[e].x + u[e].y * w[e].y;
-          q2 = r[e].x * r[e].x + r[e].y * r[e].y;
+          q0 = node_dot(r[e], u[e]);
+          q1 = node_dot(u[e], w[e]);
+          q2 = node_sq(r[e]);
         }
         double *q = sq + 64 * j + 32 * e + lane;
         q[0] = q0;

@@ -79,6 +79,14 @@ template <typename T> struct CgGeom {
 // columns, so refills never wait for a consumer warp's arithmetic
 constexpr int CG_THREADS = (WPC + 1) * 32;
 
+// A node's terms of the sums r.u, w.u and ||r||^2. Which product is rounded by
+// itself is written out: left to the compiler, this kernel and the resident solve
+// (k_cgres) chose differently for ||r||^2, and the sums differed in their last bit.
+__device__ __forceinline__ double node_dot(double2 a, double2 b) {
+  return fma(a.x, b.x, a.y * b.y);
+}
+__device__ __forceinline__ double node_sq(double2 a) { return fma(a.y, a.y, a.x * a.x); }
+
 // One launch, columns from left to right or (REV: odd phases of TURN) from right to left.
 template <typename T, typename C, int PRE, int NG, bool REV>
 __device__ __forceinline__ void cg_run(const CgArgs &A, int L, unsigned char *smem,
@@ -243,8 +251,8 @@ __device__ __forceinline__ void cg_run(const CgArgs &A, int L, unsigned char *sm
         } else {
           st2<T>(pv, o, mk2<T>(T(un.x), T(un.y)));  // p_0 = u_0
         }
-        acc[0] += (double)rc.x * un.x + (double)rc.y * un.y;
-        acc[2] += (double)rc.x * rc.x + (double)rc.y * rc.y;
+        acc[0] += node_dot(rc, un);
+        acc[2] += node_sq(rc);
       }
     }
     const V2<C> uu = shfl_down2<C>(un);  // u at (c, y+1)
@@ -273,7 +281,7 @@ __device__ __forceinline__ void cg_run(const CgArgs &A, int L, unsigned char *sm
       if (m_prev & FIXED_Y) wv.y = un_prev.y;
       const V2<T> wt = mk2<T>(T(wv.x), T(wv.y));
       st2<T>(w_out, slot_of(xo), wt);
-      acc[1] += (double)un_prev.x * (double)wt.x + (double)un_prev.y * (double)wt.y;
+      acc[1] += node_dot(un_prev, wt);
     }
     carry = REV ? fbl : mk2<C>(fbr.x + tr_below.x, fbr.y + tr_below.y);
     if (REV) carry2 = tl_below;
