@@ -1,55 +1,18 @@
 """libtpo's host code on a machine of two devices: launch attributes belong to
 the device that was current when they were set, so every device a process uses
 needs its own, and a device that cannot give the resident solve what it needs
-still solves. The library is compiled against a CUDA runtime over host memory
-(fake_cuda/runtime.cpp) that checks each launch and logs it; nothing runs.
+still solves. On a CUDA runtime over host memory (conftest.host_lib).
 """
 
 import ctypes
-import subprocess
-from pathlib import Path
 
 import numpy as np
 import pytest
 
-from conftest import REPO
+from conftest import host_launches
 from toptimization_b200 import _lib
-from toptimization_b200.csrc import build
 
-SRC = REPO / "tests" / "fake_cuda" / "runtime.cpp"
 OPT_IN = 227 * 1024
-
-
-@pytest.fixture(scope="session")
-def host_build(tmp_path_factory):
-    """The library's host code with device code left as text (unoptimised: it never runs)."""
-    d = tmp_path_factory.mktemp("fake_cuda")
-    nvcc = build.nvcc()
-    subprocess.run([nvcc, "-gencode", "arch=compute_100a,code=compute_100a", "-O0", "-Xcicc", "-O0",
-                    "-std=c++17", "-Xcompiler", "-fPIC", f"-I{REPO / 'include'}", "-c", "-o",
-                    str(d / "api.o"), str(build.CSRC / "api.cu")], check=True)
-    # -Bsymbolic: the runtime of this library, whatever else the process has loaded
-    subprocess.run(["g++", "-std=c++17", "-fPIC", "-shared", "-Wl,-Bsymbolic",
-                    f"-I{Path(nvcc).resolve().parent.parent / 'include'}", "-o",
-                    str(d / "libtpo_host.so"), str(SRC), str(d / "api.o")], check=True)
-    return d / "libtpo_host.so"
-
-
-_loads = iter(range(1000))
-
-
-@pytest.fixture
-def lib(host_build, tmp_path):
-    """A fresh copy each time: the library keeps what it learnt about a device."""
-    copy = tmp_path / f"libtpo_host{next(_loads)}.so"
-    copy.write_bytes(host_build.read_bytes())
-    L = ctypes.CDLL(str(copy))
-    for name, (res, args) in _lib._SIGS.items():
-        fn = getattr(L, name)
-        fn.restype, fn.argtypes = res, args
-    L.fake_log.restype = ctypes.c_char_p
-    L.fake_limits.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_size_t]
-    return L
 
 
 def _on(L, dev):
@@ -85,12 +48,7 @@ def _solve(L, nx, ny, pre="jacobi", asynchronous=False, precision=0, recurrence=
         res = _lib.TpoSolveResult()
         rc = L.tpo_pcg_solve(g, c, p(rho), p(f), p(fixed), p(u), p(ws), ws.size,
                              ctypes.byref(res), None)
-    launches = []
-    for line in L.fake_log().decode().splitlines():
-        dev, name, *kv = line.split()
-        launches.append({"dev": int(dev), "name": name,
-                         **{k: int(v) for k, v in (x.split("=") for x in kv)}})
-    return rc, launches
+    return rc, host_launches(L)
 
 
 def _named(launches, kernel):
@@ -104,40 +62,40 @@ SIZES = [(13, 13), (97, 41), (151, 49), (400, 200), (460, 270), (900, 900)]
 
 @pytest.mark.parametrize("asynchronous", [False, True])
 @pytest.mark.parametrize("pre", ["none", "jacobi", "nodal_block_jacobi"])
-def test_every_device_of_a_process_solves(lib, pre, asynchronous):
+def test_every_device_of_a_process_solves(host_lib, pre, asynchronous):
     for nx, ny in SIZES:
         seen = []
         for dev in (0, 1, 0):
-            _on(lib, dev)
-            rc, launches = _solve(lib, nx, ny, pre, asynchronous)
-            assert rc == 0, lib.tpo_last_error_string()
+            _on(host_lib, dev)
+            rc, launches = _solve(host_lib, nx, ny, pre, asynchronous)
+            assert rc == 0, host_lib.tpo_last_error_string()
             assert launches and all(x["dev"] == dev and x["err"] == 0 for x in launches)
             assert bool(_named(launches, "k_cgres")) == (nx * ny < 500_000)
             seen.append([{k: v for k, v in x.items() if k != "dev"} for x in launches])
         assert seen[0] == seen[1] == seen[2]
 
 
-def test_cluster_size_is_each_devices_own(lib):
-    lib.fake_limits(1, 8, OPT_IN)  # no room for 16 CTAs in a cluster of device 1
+def test_cluster_size_is_each_devices_own(host_lib):
+    host_lib.fake_limits(1, 8, OPT_IN)  # no room for 16 CTAs in a cluster of device 1
     for dev, most in ((0, 16), (1, 8), (0, 16)):
-        _on(lib, dev)
+        _on(host_lib, dev)
         sizes = []
         for nx, ny in SIZES[:-1]:
-            rc, launches = _solve(lib, nx, ny)
-            assert rc == 0, lib.tpo_last_error_string()
+            rc, launches = _solve(host_lib, nx, ny)
+            assert rc == 0, host_lib.tpo_last_error_string()
             (k,) = _named(launches, "k_cgres")
             assert k["err"] == 0
             sizes.append(k["cluster"])
         assert max(sizes) > 8 if most == 16 else 1 < max(sizes) <= 8
 
 
-def test_device_without_the_shared_memory_solves_with_a_launch_per_iteration(lib):
-    lib.fake_limits(1, 16, 48 * 1024)
+def test_device_without_the_shared_memory_solves_with_a_launch_per_iteration(host_lib):
+    host_lib.fake_limits(1, 16, 48 * 1024)
     for dev, resident in ((1, False), (0, True), (1, False)):
-        _on(lib, dev)
+        _on(host_lib, dev)
         for nx, ny in SIZES[:-1]:
-            rc, launches = _solve(lib, nx, ny)
-            assert rc == 0, lib.tpo_last_error_string()
+            rc, launches = _solve(host_lib, nx, ny)
+            assert rc == 0, host_lib.tpo_last_error_string()
             assert all(x["err"] == 0 for x in launches)
             assert bool(_named(launches, "k_cgres")) == resident
             assert bool(_named(launches, "k_cgstep")) != resident
@@ -145,11 +103,11 @@ def test_device_without_the_shared_memory_solves_with_a_launch_per_iteration(lib
 
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("pre", list(_lib.PRECOND))
-def test_two_launch_forms_on_every_device(lib, pre, precision):
+def test_two_launch_forms_on_every_device(host_lib, pre, precision):
     for dev in (0, 1):
-        _on(lib, dev)
+        _on(host_lib, dev)
         for asynchronous in (False, True):
-            rc, launches = _solve(lib, 400, 200, pre, asynchronous, precision, recurrence=1)
-            assert rc == 0, lib.tpo_last_error_string()
+            rc, launches = _solve(host_lib, 400, 200, pre, asynchronous, precision, recurrence=1)
+            assert rc == 0, host_lib.tpo_last_error_string()
             assert launches and all(x["dev"] == dev and x["err"] == 0 for x in launches)
             assert not _named(launches, "k_cgres") and not _named(launches, "k_cgstep")

@@ -1898,13 +1898,14 @@ static int filter_launch(const tpo_grid *g, double rmin, int mode, const double 
   const double den = filter_den(rmin, R);
   const dim3 gr((g->nely + FT - 1) / FT, (g->nelx + FT - 1) / FT, 1);
   cudaStream_t st = static_cast<cudaStream_t>(s);
-  if (mode == F_DENSITY) {
-    k_filter<F_DENSITY><<<gr, F_THREADS, smem, st>>>(g->nelx, g->nely, rmin, R, x, rho, out, s_out,
-                                                     s32_out, g->e_min, g->penalty, den);
-  } else {
-    k_filter<F_SENS><<<gr, F_THREADS, smem, st>>>(g->nelx, g->nely, rmin, R, x, rho, out, nullptr,
-                                                  nullptr, g->e_min, g->penalty, den);
-  }
+  const bool dens = mode == F_DENSITY;
+  if (!dens) s_out = nullptr, s32_out = nullptr;
+  if (R > F_REGR)
+    (dens ? k_filter_any<F_DENSITY> : k_filter_any<F_SENS>)<<<gr, FA_THREADS, smem, st>>>(
+        g->nelx, g->nely, rmin, R, x, rho, out, s_out, s32_out, g->e_min, g->penalty);
+  else
+    (dens ? k_filter<F_DENSITY> : k_filter<F_SENS>)<<<gr, F_THREADS, smem, st>>>(
+        g->nelx, g->nely, rmin, R, x, rho, out, s_out, s32_out, g->e_min, g->penalty, den);
   TPO_CK_LAUNCH();
   return TPO_OK;
 }

@@ -88,8 +88,10 @@ __device__ __forceinline__ const BJob &find_job(const BJob *__restrict__ jobs, i
 }
 
 // ---------------------------------------------------------------- kernels
-// density filter (which = 0: rho -> rho_phys) or dc filter (which = 1: dc -> dc_filt)
-__global__ void __launch_bounds__(F_THREADS)
+// density filter (which = 0: rho -> rho_phys) or dc filter (which = 1: dc -> dc_filt),
+// of designs with radii up to F_REGR or (ANY) beyond: each form has its own job table
+template <bool ANY>
+__global__ void __launch_bounds__(ANY ? FA_THREADS : F_THREADS)
     kb_filter(const BJob *jobs, int nj, const BDesign *ds, int which) {
   const BJob &J = find_job(jobs, nj);
   const BDesign &D = ds[J.slot];
@@ -97,8 +99,12 @@ __global__ void __launch_bounds__(F_THREADS)
   const int loc = blockIdx.x - J.cta0;
   const double *x = which ? D.dc : D.rho;
   double *out = which ? D.dc_filt : D.rho_phys;
-  filter_run<F_DENSITY>(D.nx, D.ny, D.rmin, D.R, x, nullptr, out, nullptr, nullptr, 0.0, 0.0, D.fden,
-                        loc % J.gx, loc / J.gx);
+  if constexpr (ANY)
+    filter_any<F_DENSITY>(D.nx, D.ny, D.rmin, D.R, x, nullptr, out, nullptr, nullptr, 0.0, 0.0,
+                          loc % J.gx, loc / J.gx);
+  else
+    filter_run<F_DENSITY>(D.nx, D.ny, D.rmin, D.R, x, nullptr, out, nullptr, nullptr, 0.0, 0.0,
+                          D.fden, loc % J.gx, loc / J.gx);
 }
 
 __global__ void kb_scales(const BJob *jobs, int nj, const BDesign *ds) {

@@ -31,7 +31,7 @@ struct tpo_batch {
   // launch state
   bool dirty = true;
   int njobs[8]{}, nctas[8]{};
-  int filter_smem = 0;
+  int filter_smem[2] = {0, 0};  // radii up to F_REGR, beyond
   int Ls = 16, Lu = 8;          // strip lengths (columns per CTA) of the stencil / update kinds
   int round_steps = 32;         // PCG steps per round
   cudaGraphExec_t gexec = nullptr;   // OC-iteration graph
@@ -45,7 +45,7 @@ namespace {
 using tpo::BDesign;
 using tpo::BJob;
 
-enum BKind { BK_FILTER = 0, BK_SCALES, BK_UNPACK, BK_STENCIL, BK_UPDATE, BK_SENS, kBK };
+enum BKind { BK_FILTER = 0, BK_FILTER_ANY, BK_SCALES, BK_UNPACK, BK_STENCIL, BK_UPDATE, BK_SENS, kBK };
 constexpr int kBatchSteps = 8;       // PCG steps per loop body (one FP64 residual check each)
 constexpr int kFlatPerThread = 4;    // elements per thread of the grid-stride kinds
 
@@ -61,6 +61,7 @@ void kind_geom(int kind, int nx, int ny, int P, int Ls, int Lu, int *gx, int *gy
   *L = 0;
   switch (kind) {
     case BK_FILTER:
+    case BK_FILTER_ANY:
       *gx = cdiv(ny, FT);
       *gy = cdiv(nx, FT);
       break;
@@ -163,7 +164,7 @@ template <int PRE> int batch_set_attrs() {
   constexpr int SMEM_D = TsGeom<float, M_DIR>::template slot_bytes<kBatchG>() * kBatchNG;
   TPO_CK(cudaFuncSetAttribute(kb_resx<PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
   TPO_CK(cudaFuncSetAttribute(kb_dir<PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_D));
-  TPO_CK(cudaFuncSetAttribute(kb_filter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  TPO_CK(cudaFuncSetAttribute(kb_filter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               filter_smem_bytes(F_MAXR)));
   return TPO_OK;
 }
@@ -171,28 +172,31 @@ template <int PRE> int batch_set_attrs() {
 // rebuild the job tables of every kind from the active slots
 int batch_rebuild(tpo_batch *b, cudaStream_t st) {
   std::vector<BJob> h((size_t)kBK * b->max_designs);
-  int fsm = 0;
+  int fsm[2] = {0, 0};
   unsigned mb = 4;
   for (int k = 0; k < kBK; ++k) {
     int n = 0, cta = 0;
     for (int s = 0; s < b->n_slots; ++s) {
       if (!b->used[s] || !b->h_status[2 * s + 1]) continue;
       const BDesign &D = b->rec[s];
+      const bool any = D.R > F_REGR;
+      if (k == (any ? BK_FILTER : BK_FILTER_ANY)) continue;
       BJob j{};
       kind_geom(k, D.nx, D.ny, D.P, b->Ls, b->Lu, &j.gx, &j.gy, &j.L);
       j.cta0 = cta;
       j.slot = s;
       cta += j.gx * j.gy;
       h[(size_t)k * b->max_designs + n++] = j;
-      if (k == 0) {
-        fsm = std::max(fsm, filter_smem_bytes(D.R));
+      if (k == BK_SCALES) {
+        fsm[any] = std::max(fsm[any], filter_smem_bytes(D.R));
         mb = std::max(mb, (unsigned)(D.max_cg + D.max_outer + 4));
       }
     }
     b->njobs[k] = n;
     b->nctas[k] = cta;
   }
-  b->filter_smem = fsm;
+  b->filter_smem[0] = fsm[0];
+  b->filter_smem[1] = fsm[1];
   b->max_bodies = mb;
   TPO_CK(cudaMemcpyAsync(b->d_jobs, h.data(), h.size() * sizeof(BJob), cudaMemcpyHostToDevice, st));
   TPO_CK(cudaStreamSynchronize(st));
@@ -216,12 +220,24 @@ const BJob *jobs_of(const tpo_batch *b, int kind) {
   return b->d_jobs + (size_t)kind * b->max_designs;
 }
 
+int batch_filter(tpo_batch *b, cudaStream_t st, int which) {
+  if (b->nctas[BK_FILTER]) {
+    kb_filter<false><<<b->nctas[BK_FILTER], F_THREADS, b->filter_smem[0], st>>>(
+        jobs_of(b, BK_FILTER), b->njobs[BK_FILTER], b->d_designs, which);
+    TPO_CK_LAUNCH();
+  }
+  if (b->nctas[BK_FILTER_ANY]) {
+    kb_filter<true><<<b->nctas[BK_FILTER_ANY], FA_THREADS, b->filter_smem[1], st>>>(
+        jobs_of(b, BK_FILTER_ANY), b->njobs[BK_FILTER_ANY], b->d_designs, which);
+    TPO_CK_LAUNCH();
+  }
+  return TPO_OK;
+}
+
 // launches of one OC iteration, before and after the PCG loop
 int batch_prefix(tpo_batch *b, cudaStream_t st) {
-  if (b->nctas[BK_FILTER] == 0) return TPO_OK;
-  kb_filter<<<b->nctas[BK_FILTER], F_THREADS, b->filter_smem, st>>>(
-      jobs_of(b, BK_FILTER), b->njobs[BK_FILTER], b->d_designs, 0);
-  TPO_CK_LAUNCH();
+  if (b->nctas[BK_SCALES] == 0) return TPO_OK;
+  if (int rc = batch_filter(b, st, 0)) return rc;
   kb_scales<<<b->nctas[BK_SCALES], 256, 0, st>>>(jobs_of(b, BK_SCALES), b->njobs[BK_SCALES],
                                                   b->d_designs);
   TPO_CK_LAUNCH();
@@ -268,9 +284,7 @@ int batch_suffix(tpo_batch *b, cudaStream_t st) {
   kb_sens<<<b->nctas[BK_SENS], S_THREADS, 0, st>>>(jobs_of(b, BK_SENS), b->njobs[BK_SENS],
                                                      b->d_designs);
   TPO_CK_LAUNCH();
-  kb_filter<<<b->nctas[BK_FILTER], F_THREADS, b->filter_smem, st>>>(
-      jobs_of(b, BK_FILTER), b->njobs[BK_FILTER], b->d_designs, 1);
-  TPO_CK_LAUNCH();
+  if (int rc = batch_filter(b, st, 1)) return rc;
   kb_oc<<<b->n_slots * kClusterCtas, OC_THREADS, 0, st>>>(b->d_designs, b->n_slots);
   TPO_CK_LAUNCH();
   kb_finish<<<cdiv(b->n_slots, 128), 128, 0, st>>>(b->d_designs, b->n_slots, b->d_status,
@@ -619,7 +633,7 @@ int tpo_batch_oc_iteration(tpo_batch *b, tpo_stream s) {
   cudaStream_t st = static_cast<cudaStream_t>(s);
   int rc;
   if (b->dirty && (rc = batch_rebuild(b, st))) return rc;
-  if (b->nctas[BK_FILTER] == 0) return TPO_OK;  // nothing active
+  if (b->nctas[BK_SCALES] == 0) return TPO_OK;  // nothing active
   if (b->cfg.use_graph) {
     if (!b->gexec && (rc = batch_build_graph(b))) return rc;
     TPO_CK(cudaGraphLaunch(b->gexec, st));
@@ -636,7 +650,7 @@ int tpo_batch_round(tpo_batch *b, int32_t rounds, tpo_stream s) {
   cudaStream_t st = static_cast<cudaStream_t>(s);
   int rc;
   if (b->dirty && (rc = batch_rebuild(b, st))) return rc;
-  if (b->nctas[BK_FILTER] == 0) return TPO_OK;
+  if (b->nctas[BK_SCALES] == 0) return TPO_OK;
   for (int i = 0; i < rounds; ++i) {
     if (b->cfg.use_graph) {
       if (!b->rexec && (rc = batch_build_round_graph(b))) return rc;
@@ -666,7 +680,7 @@ int tpo_batch_time_steps(tpo_batch *b, int32_t steps, tpo_stream s, float *ms_ou
   cudaStream_t st = static_cast<cudaStream_t>(s);
   int rc;
   if (b->dirty && (rc = batch_rebuild(b, st))) return rc;
-  if (b->nctas[BK_FILTER] == 0) return fail(TPO_ERR_ARGS, "no active design");
+  if (b->nctas[BK_SCALES] == 0) return fail(TPO_ERR_ARGS, "no active design");
   if ((rc = batch_prefix(b, st))) return rc;
   if ((rc = batch_body_any(b, st, 0, 0))) return rc;  // FP64 residual, first steps
   // the events are released on every path out of the timed region

@@ -17,12 +17,19 @@ namespace tpo {
 // (dx outer, dy inner), skipping w <= 0 and out-of-domain neighbours.
 // ---------------------------------------------------------------------------
 constexpr int FT = 32;           // tile edge (elements)
-constexpr int F_THREADS = 128;
+constexpr int F_THREADS = 128;   // radii up to F_REGR
+constexpr int FA_THREADS = 256;  // larger radii
+constexpr int F_REGR = 8;
 constexpr int F_MAXR = 16;
 
 enum FilterMode { F_DENSITY = 0, F_SENS = 1 };
 
-// Any radius up to F_MAXR. (bx, by) = (tile row, tile column) of this CTA
+// Radii from F_REGR + 1 to F_MAXR. (bx, by) = (tile row, tile column) of this CTA.
+// Bound by two shared loads and two tests per neighbour and by the warps that cover
+// their latency: a tile of 21 to 41 KB limits the CTAs of an SM, so a CTA has 256
+// threads, in a kernel without the register form's 78 registers. Density filter of
+// 517x173 elements at R = 9, 12, 16: 40, 61, 96 us (47, 67, 105 without the unrolled
+// row; 80, 114, 179 with 128 threads and both forms in one kernel).
 template <int MODE>
 __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
                                            const double *__restrict__ x,
@@ -55,7 +62,7 @@ __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
 
   const int ty = threadIdx.x & 31;
   const int ey = ey0 + ty;
-  for (int tx = threadIdx.x >> 5; tx < FT; tx += F_THREADS / 32) {
+  for (int tx = threadIdx.x >> 5; tx < FT; tx += FA_THREADS / 32) {
     const int ex = ex0 + tx;
     if (ex >= nx || ey >= ny) continue;
     double num = 0.0, den = 0.0;
@@ -64,6 +71,7 @@ __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
       if (jx < 0 || jx >= nx) continue;
       const double *trow = tile + (size_t)(tx + R + dx) * TW + (ty + R);
       const double *wrow = wt + (dx + R) * W + R;
+#pragma unroll 4
       for (int dy = -R; dy <= R; ++dy) {
         const double w = wrow[dy];
         const int jy = ey + dy;
@@ -96,7 +104,6 @@ __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
 // whose box lies inside the grid takes the weight sum den_in (filter_den).
 // Values and weights are added in the reference's order (dx, then dy). At rmin = 4
 // on 2048x1024 elements 96 -> 33 us (46 us with the tile staged one load at a time).
-constexpr int F_REGR = 8;
 constexpr int F_ROWS = 8;
 static_assert(F_THREADS / 32 * F_ROWS == FT, "a CTA covers the tile");
 template <int MODE, int R>
@@ -243,7 +250,6 @@ __device__ __forceinline__ void filter_run(int nx, int ny, double rmin, int R,
     break;
     TPO_F(1) TPO_F(2) TPO_F(3) TPO_F(4) TPO_F(5) TPO_F(6) TPO_F(7) TPO_F(8)
 #undef TPO_F
-    default: filter_any<MODE>(nx, ny, rmin, R, x, rho, out, s_out, s32_out, e_min, pen, bx, by);
   }
 }
 template <int MODE>
@@ -253,6 +259,15 @@ __global__ void __launch_bounds__(F_THREADS)
              double *__restrict__ s_out, float *__restrict__ s32_out, double e_min, double pen,
              double den) {
   filter_run<MODE>(nx, ny, rmin, R, x, rho, out, s_out, s32_out, e_min, pen, den, blockIdx.x,
+                   blockIdx.y);
+}
+template <int MODE>
+__global__ void __launch_bounds__(FA_THREADS)
+    k_filter_any(int nx, int ny, double rmin, int R, const double *__restrict__ x,
+                 const double *__restrict__ rho, double *__restrict__ out,
+                 double *__restrict__ s_out, float *__restrict__ s32_out, double e_min,
+                 double pen) {
+  filter_any<MODE>(nx, ny, rmin, R, x, rho, out, s_out, s32_out, e_min, pen, blockIdx.x,
                    blockIdx.y);
 }
 
