@@ -1894,7 +1894,7 @@ static int filter_launch(const tpo_grid *g, double rmin, int mode, const double 
   if (!(rmin > 0.0)) return fail(TPO_ERR_ARGS, "rmin must be > 0");
   const int R = (int)std::ceil(rmin);
   if (R > F_MAXR) return fail(TPO_ERR_ARGS, "ceil(rmin) = %d exceeds %d", R, F_MAXR);
-  const size_t smem = (size_t)filter_smem_bytes(R);
+  const size_t smem = (size_t)filter_smem_bytes(R, mode);
   const double den = filter_den(rmin, R);
   const dim3 gr((g->nely + FT - 1) / FT, (g->nelx + FT - 1) / FT, 1);
   cudaStream_t st = static_cast<cudaStream_t>(s);

@@ -119,6 +119,7 @@ __device__ __forceinline__ void filter_reg(int nx, int ny, double rmin,
   extern __shared__ __align__(16) double fsm[];
   double *tile = fsm;               // [TC][PITCH], rows from ey0 - RA
   double *wt = fsm + TC * PITCH;    // [R + 1][R + 1] by |dx|, |dy|
+  double *own = wt + (R + 1) * (R + 1);  // F_SENS: rho of the tile itself, [FT][FT + 1]
   __shared__ int chord[R + 1];      // largest |dy| with a positive weight (-1: none)
   const int ex0 = by * FT, ey0 = bx * FT;
   for (int k = threadIdx.x; k < (R + 1) * (R + 1); k += F_THREADS) {
@@ -133,21 +134,27 @@ __device__ __forceinline__ void filter_reg(int nx, int ny, double rmin,
   }
   constexpr int NB = 8;  // loads in flight per thread
   for (int k0 = threadIdx.x; k0 < TC * TH; k0 += NB * F_THREADS) {
-    double v[NB];
+    double v[NB], q[MODE == F_SENS ? NB : 1];
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
       const int k = k0 + i * F_THREADS, tx = k / TH, ty = k - tx * TH;
       const int gx = ex0 - R + tx, gy = ey0 - RA + ty;
       v[i] = 0.0;
+      if (MODE == F_SENS) q[i] = 0.0;
       if (k < TC * TH && gx >= 0 && gx < nx && gy >= 0 && gy < ny) {
         const size_t e = (size_t)gx * ny + gy;
-        v[i] = (MODE == F_SENS) ? rho[e] * x[e] : x[e];
+        v[i] = x[e];
+        if (MODE == F_SENS) q[i] = rho[e];
       }
     }
 #pragma unroll
     for (int i = 0; i < NB; ++i) {
       const int k = k0 + i * F_THREADS, tx = k / TH, ty = k - tx * TH;
-      if (k < TC * TH) tile[tx * PITCH + ty] = v[i];
+      if (k < TC * TH) {
+        tile[tx * PITCH + ty] = MODE == F_SENS ? q[i] * v[i] : v[i];
+        if (MODE == F_SENS && (unsigned)(tx - R) < FT && (unsigned)(ty - RA) < FT)
+          own[(tx - R) * (FT + 1) + ty - RA] = q[i];
+      }
     }
   }
   __syncthreads();
@@ -204,7 +211,7 @@ __device__ __forceinline__ void filter_reg(int nx, int ny, double rmin,
     const size_t e = (size_t)ex * ny + yj;
     double o;
     if (MODE == F_SENS) {
-      o = num[j] / (rho[e] * den[j] + 1e-20);
+      o = num[j] / (own[tx * (FT + 1) + r0 + j] * den[j] + 1e-20);
     } else {
       o = num[j] / (den[j] + 1e-20);
       if (s_out || s32_out) {
@@ -229,10 +236,11 @@ inline double filter_den(double rmin, int R) {
 }
 
 // dynamic shared memory of a filter launch
-inline int filter_smem_bytes(int R) {
+inline int filter_smem_bytes(int R, int mode = F_DENSITY) {
   const int W = 2 * R + 1, TW = FT + 2 * R, RA = (R + 1) / 2 * 2;
   if (R > F_REGR) return (W * W + TW * TW) * (int)sizeof(double);
-  return (TW * (FT + 2 * RA + 2) + (R + 1) * (R + 1)) * (int)sizeof(double);
+  const int own = mode == F_SENS ? FT * (FT + 1) : 0;
+  return (TW * (FT + 2 * RA + 2) + (R + 1) * (R + 1) + own) * (int)sizeof(double);
 }
 
 template <int MODE>
