@@ -288,10 +288,15 @@ __global__ void __launch_bounds__(FA_THREADS)
 // 1200 elements (80 us at 2048x1024). The dense product keeps the
 // order of its sums: uKu cancels from |u|^2 down to the squared strains, so
 // another order moves dc by 1e-11 on a 2048-element span.
+// The product is a function call: inlined, the loop keeps Ke's 64 entries in 128
+// registers (or, held at 64, spills them: 276 bytes a thread), where the function
+// takes them as constant operands and leaves 48. Inlined and spilled / inlined at
+// 128 registers / called: 69.9, 51.9, 40.0 us at 2048x1024, 24.4, 18.6, 14.4 at
+// 3x100000 (the column march of before: 65.7, 20.6).
 // ---------------------------------------------------------------------------
 constexpr int S_THREADS = 256;
 
-__device__ __forceinline__ double elem_energy(double2 bl, double2 br, double2 tr, double2 tl) {
+__device__ __noinline__ double elem_energy(double2 bl, double2 br, double2 tr, double2 tl) {
   const double ue[8] = {bl.x, bl.y, br.x, br.y, tr.x, tr.y, tl.x, tl.y};
   double uku = 0.0;
 #pragma unroll
@@ -323,7 +328,7 @@ __device__ __forceinline__ void sensitivity_run(int nx, int ny, double e_min, do
   if (!grid_reduce<1>(acc, part, &ctl->counter, nb, bid)) return;
   if (threadIdx.x == 0) *c_out = acc[0];
 }
-__global__ void __launch_bounds__(S_THREADS, 4)
+__global__ void __launch_bounds__(S_THREADS, 5)
     k_sensitivity(int nx, int ny, double e_min, double pen, const double *__restrict__ rho,
                   const double *__restrict__ u, double *__restrict__ dc, double *part,
                   SumCtl *ctl, double *c_out) {
