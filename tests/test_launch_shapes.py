@@ -24,3 +24,17 @@ def test_large_filter_radii_have_256_threads_per_tile(host_lib, rmin, sens):
     assert rc == 0, host_lib.tpo_last_error_string()
     (k,) = host_launches(host_lib)
     assert k["err"] == 0 and k["threads"] == 256 and k["grid"] == 3 * 2
+
+
+@pytest.mark.parametrize("rmin,kernel", [(0.9, "taps<0,27>"), (1.0, "taps<0,27>"),
+                                         (2.0, "taps<0,27>"), (2.1, "taps<0,304>"),
+                                         (4.1, "taps<0,304>"), (4.4, "filter<0>")])
+def test_filter3_argument_no_larger_than_its_list(host_lib, rmin, kernel):
+    """A neighbour list is a kernel argument; a long one delays the launch."""
+    n = 9 * 8 * 7
+    a = [np.zeros(n) for _ in range(2)]
+    g = _lib.grid3(9, 8, 7, 1e-9, 3.0)
+    rc = host_lib.tpo3_density_filter(g, rmin, a[0].ctypes.data, a[1].ctypes.data, None)
+    assert rc == 0, host_lib.tpo_last_error_string()
+    (k,) = host_launches(host_lib)
+    assert k["err"] == 0 and k["name"].endswith(kernel), k["name"]

@@ -1223,22 +1223,26 @@ __global__ void __launch_bounds__(H3_FLAT)
 // 4.2: H3_TAPS neighbours). An element whose box lies inside the grid adds the
 // listed neighbours and divides by the common weight sum; the others test each
 // neighbour. The box walk above visits and tests (2 R + 1)^3 candidates per
-// element for the 19 of rmin = 1.5 (51 us at 128x64x64).
-constexpr int H3_TAPS = 304;
-struct Hex3Taps {
-  int n, reach;          // neighbours; largest |offset| along an axis
-  double den;            // sum of their weights
-  double w[H3_TAPS];
-  int8_t d[H3_TAPS][4];  // dx, dy, dz
+// element for the 19 of rmin = 1.5 (51 us at 128x64x64). Lists of up to
+// H3_FEW_TAPS (rmin up to 2) travel as an argument of a tenth of the size: the
+// larger one alone costs a launch 0.45 us, which at rmin <= 1 (the element itself)
+// on a small grid was more than the box walk cost.
+constexpr int H3_TAPS = 304, H3_FEW_TAPS = 27;
+template <int CAP> struct Hex3Taps {
+  int n, reach;      // neighbours; largest |offset| along an axis
+  double den;        // sum of their weights
+  double w[CAP];
+  int8_t d[CAP][4];  // dx, dy, dz
 };
-static_assert(sizeof(Hex3Taps) + 64 <= 4096, "kernel arguments");
+static_assert(sizeof(Hex3Taps<H3_TAPS>) + 64 <= 4096, "kernel arguments");
 
-template <int MODE>
+template <int MODE, int CAP>
 __global__ void __launch_bounds__(H3_FLAT)
-    k_hex_filter_taps(Hex3 g, const __grid_constant__ Hex3Taps t, const double *__restrict__ x,
-                      const double *__restrict__ rho, double *__restrict__ out) {
-  __shared__ double sw[H3_TAPS];
-  __shared__ int so[H3_TAPS];
+    k_hex_filter_taps(Hex3 g, const __grid_constant__ Hex3Taps<CAP> t,
+                      const double *__restrict__ x, const double *__restrict__ rho,
+                      double *__restrict__ out) {
+  __shared__ double sw[CAP];
+  __shared__ int so[CAP];
   for (int k = threadIdx.x; k < t.n; k += H3_FLAT) {
     sw[k] = t.w[k];
     so[k] = (t.d[k][0] * g.ny + t.d[k][1]) * g.nz + t.d[k][2];

@@ -311,7 +311,7 @@ Sens3Ws carve_sens3(void *base) {
 
 // the neighbours with positive weights in the order dx, dy, dz; false if they
 // are more than a launch's list holds
-bool hex_taps(double rmin, int R, Hex3Taps *t) {
+template <int CAP> bool hex_taps(double rmin, int R, Hex3Taps<CAP> *t) {
   t->n = 0;
   t->reach = 0;
   t->den = 0.0;
@@ -320,7 +320,7 @@ bool hex_taps(double rmin, int R, Hex3Taps *t) {
       for (int dz = -R; dz <= R; ++dz) {
         const double w = rmin - std::sqrt((double)(dx * dx + dy * dy + dz * dz));
         if (!(w > 0.0)) continue;
-        if (t->n == H3_TAPS) return false;
+        if (t->n == CAP) return false;
         t->w[t->n] = w;
         t->d[t->n][0] = (int8_t)dx;
         t->d[t->n][1] = (int8_t)dy;
@@ -346,15 +346,19 @@ int filter3_launch(const tpo_grid3 *g, double rmin, int mode, const double *x, c
   const Hex3 h = hex_of(g);
   cudaStream_t st = static_cast<cudaStream_t>(s);
   const dim3 gr = hex_flat_grid(h.elems());
-  Hex3Taps taps;
-  if (hex_taps(rmin, R, &taps)) {
-    if (mode == F_SENS)
-      k_hex_filter_taps<F_SENS><<<gr, H3_FLAT, 0, st>>>(h, taps, x, rho, out);
-    else
-      k_hex_filter_taps<F_DENSITY><<<gr, H3_FLAT, 0, st>>>(h, taps, x, nullptr, out);
+  auto by_list = [&](const auto &taps, auto kern) -> int {
+    kern<<<gr, H3_FLAT, 0, st>>>(h, taps, x, mode == F_SENS ? rho : nullptr, out);
     TPO_CK_LAUNCH();
     return TPO_OK;
-  }
+  };
+  Hex3Taps<H3_FEW_TAPS> few;
+  if (hex_taps(rmin, R, &few))
+    return by_list(few, mode == F_SENS ? k_hex_filter_taps<F_SENS, H3_FEW_TAPS>
+                                       : k_hex_filter_taps<F_DENSITY, H3_FEW_TAPS>);
+  Hex3Taps<H3_TAPS> taps;
+  if (hex_taps(rmin, R, &taps))
+    return by_list(taps, mode == F_SENS ? k_hex_filter_taps<F_SENS, H3_TAPS>
+                                        : k_hex_filter_taps<F_DENSITY, H3_TAPS>);
   if (mode == F_SENS)
     k_hex_filter<F_SENS><<<gr, H3_FLAT, smem, st>>>(h, rmin, R, x, rho, out);
   else
