@@ -267,8 +267,8 @@ typedef struct tpo_profile {
   double apply_ms;
   int64_t apply_bytes;
   int64_t step_launches;    /* iterations of the one-launch form (TPO_RECURRENCE_SINGLE) */
-  double step_ms;
-  int64_t step_bytes;
+  double step_ms;           /* theirs; where one launch is the whole solve, its set-up too */
+  int64_t step_bytes;       /* there: the caller's arrays once, no vectors per iteration */
 } tpo_profile;
 int tpo_profile_enable(int on);
 int tpo_profile_reset(void);

@@ -1083,6 +1083,14 @@ int launch_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, con
   return TPO_OK;
 }
 
+// What a resident solve moves through memory: densities, load, mask and starting
+// values in, the solution out. Its vectors stay on the chip, and the exchanged words
+// in shared memory or the L2.
+int64_t res_bytes(const tpo_grid *g, bool warm) {
+  const int64_t nn = (int64_t)(g->nelx + 1) * (g->nely + 1);
+  return 8 * (int64_t)g->nelx * g->nely + (warm ? 49 : 33) * nn;
+}
+
 // Blocking form: the whole solve is one launch (cluster) or two.
 template <int PRE>
 int pcg_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const double *f,
@@ -1101,7 +1109,7 @@ int pcg_res(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, const 
     TPO_CK(cudaEventElapsedTime(&ms, ev[0], ev[1]));
     g_prof.step_ms += ms;
     g_prof.step_launches += fin.it;
-    g_prof.step_bytes += (int64_t)fin.it * step_bytes<double>(g).step;
+    g_prof.step_bytes += res_bytes(g, c->warm_start != 0);
   }
   out->status = fin.status == TPO_SOLVE_RUNNING ? TPO_SOLVE_MAX_ITER : fin.status;
   out->updates = fin.it;
