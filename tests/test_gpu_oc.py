@@ -101,3 +101,17 @@ def test_lowest_midpoints_count_the_regulariser(n):
     with_, without = 0.5 * np.sqrt(lam / (lam + 1e-20)), 0.5
     assert 5e-16 < without - with_ < 2e-15
     _run(np.full(n, 0.5), np.full(n, -lam), 0.5 * (with_ + without))
+
+
+@pytest.mark.parametrize("n", [4 * 148 * 1024, 4 * 148 * 1024 + 1])
+@pytest.mark.parametrize("either_sign", [False, True])
+def test_two_levels_per_pass(n, either_sign):
+    """dv on either side of the size from which a pass takes two levels of the
+    bisection instead of three (148 SMs). The volumes' rounding, below 1e-12 of
+    them, is far from the target at every midpoint but the last few, whose
+    lambda then differ by 1e-4 at most; the seeds below do not meet that."""
+    rng = np.random.default_rng(6)
+    rho = rng.uniform(0.001, 1.0, n)
+    dc = -rng.exponential(1.0, n)
+    dv = rng.uniform(-0.5 if either_sign else 0.5, 2.0, n)
+    _run(rho, dc, 0.4, dv=dv)

@@ -361,11 +361,18 @@ __global__ void __launch_bounds__(S_THREADS, 5)
 // from 1e9 / 2^43 down, the 43rd midpoint, it is part of the sum.) s stays
 // in registers (up to OC_EPT elements per thread) or in `sbuf` (n doubles).
 // The density, its mean and the largest change come from the formula itself.
+// With dv every value of lambda costs a division and a square root, and on large
+// designs their number is the time, not the passes. Beyond OC_DV_EPT elements per
+// thread a pass evaluates two levels of the tree: 75 values in 25 passes instead of
+// 119 in 17. Two levels / three: 176, 154 us at 303,104 elements, 221, 226 at 500,000,
+// 248, 257 at 700,000, 471, 577 at 2.1 M, 1.75, 2.12 ms at 8 M, 6.3, 8.0 ms at 32 M
+// (7.7 there with a launch per midpoint).
 // ---------------------------------------------------------------------------
 constexpr int OC_THREADS = 1024;
 constexpr int OC_MAX_STEPS = 50;
 constexpr int OC_NL = 7;
 constexpr int OC_EPT = 2;
+constexpr int OC_DV_EPT = 4;
 
 __device__ __forceinline__ double oc_candidate(double r, double d, double dvv, double lam,
                                                double move) {
@@ -405,8 +412,8 @@ struct OcWalk {
       default: return 0.5 * (mh + hi);
     }
   }
-  // above: bit j set if the volume at value j exceeds the target
-  __device__ __forceinline__ void walk(unsigned above) {
+  // above: bit j set if the volume at value j exceeds the target; levels: of the tree, evaluated
+  __device__ __forceinline__ void walk(unsigned above, int levels) {
     if (scan == 1) {
       const int j = above ? __ffs(above) - 1 : OC_NL;
       k0 = OC_NL * j;
@@ -446,7 +453,7 @@ struct OcWalk {
     for (int i = 0; i < 3; ++i) stop[i] = (h[i] - l[i]) / (h[i] + l[i] + 1e-30) < 1e-4;
 #pragma unroll
     for (int i = 0; i < 3; ++i)
-      if (!done) {
+      if (i < levels && !done) {
         lo = l[i];
         hi = h[i];
         last = m[i];
@@ -472,6 +479,7 @@ __device__ __forceinline__ void oc_run(Team &team, int n, double volfrac, double
                                        const double *__restrict__ dv, double *sbuf,
                                        double *rho_out, double *result, OcShared &sh) {
   const int stride = team.size() * OC_THREADS;
+  const int levels = !HELD && dv && n > OC_DV_EPT * stride ? 2 : 3;
   const int e0 = team.rank() * OC_THREADS + threadIdx.x;
   double hr[HELD ? OC_EPT : 1], hs[HELD ? OC_EPT : 1];
   if (HELD) {
@@ -494,7 +502,7 @@ __device__ __forceinline__ void oc_run(Team &team, int n, double volfrac, double
       OcWalk w = sh.w;
       const unsigned above =
           __ballot_sync(FULL, sum && threadIdx.x < OC_NL && sum[threadIdx.x] / n > volfrac);
-      if (sum) w.walk(above);
+      if (sum) w.walk(above, levels);
       else w.init(dv == nullptr);
       if (threadIdx.x == 0) sh.w = w;
       if (threadIdx.x < OC_NL) {
@@ -524,7 +532,8 @@ __device__ __forceinline__ void oc_run(Team &team, int n, double volfrac, double
       for (int e = e0; e < n; e += stride) {
         const double r = rho_in[e], d = dc[e], v = dv[e];
 #pragma unroll
-        for (int j = 0; j < OC_NL; ++j) acc[j] += oc_candidate(r, d, v, il[j], move);
+        for (int j = 0; j < OC_NL; ++j)
+          if (j < 3 || levels == 3) acc[j] += oc_candidate(r, d, v, il[j], move);
       }
     } else if (HELD) {
 #pragma unroll
