@@ -74,7 +74,7 @@ enum {
 /* PCG recurrence. AUTO: one launch per iteration (Chronopoulos-Gear form,
  * one global reduction) for the plain FP64 solve with a point preconditioner
  * (none, Jacobi, nodal block), or one for the whole solve where the grid fits
- * the chip (about 140,000 nodes; the same bits); two launches otherwise (element-block
+ * the chip (142,080 nodes at most; the same bits); two launches otherwise (element-block
  * preconditioner, mixed form). STANDARD: the reference's own recurrence
  * (fem/solver.py:27-159), two launches per iteration. SINGLE: AUTO's first
  * form; TPO_ERR_ARGS for the element-block preconditioner or the mixed form
@@ -180,7 +180,7 @@ int tpo_pcg_solve(const tpo_grid *g, const tpo_solve_cfg *c,
  * runs on the device as a CUDA graph conditional WHILE node (bodies of 16
  * iterations, the stop, breakdown and refinement rules decided by the
  * kernels, a bound on the number of bodies) or, where the grid fits the chip,
- * inside one kernel (no graph, no bodies), and the result is written to
+ * inside one kernel (no WHILE node, no bodies), and the result is written to
  * `out_dev`, DEVICE memory (8-byte aligned), when the solve has finished.
  * Same kernels in the same order as tpo_pcg_solve, so the same results.
  * If `s` is capturing, the solve's nodes are added to that capture (so a

@@ -906,12 +906,17 @@ int pcg_mixed(const tpo_grid *g, const tpo_solve_cfg *c, const double *rho, cons
 
 // ----------------------------------------------------------------- resident PCG
 // Plan of the resident solve (k_cgres): k_cgstep's strips in groups of 30 rows.
-// One cluster if 16 CTAs hold the groups (its exchange takes about 1 us less
-// than polled words), otherwise one CTA per SM at most; the fewest groups per
-// CTA that allow it; none if 640 threads do not hold them.
+// One cluster if 16 CTAs hold the groups, one or two each (its exchange takes about
+// 1 us less than polled words), otherwise one CTA per SM at most; the fewest groups
+// per CTA that allow it; none if 640 threads do not hold them.
 // Measured per iteration, against 13-16 us with one launch each:
-//   cluster:     60x20 2.3 us, 97x41 2.8
-//   cooperative: 151x49 3.9, 200x100 4.5, 400x200 6.8 (17 before), 460x270 8.5 (19)
+//   cluster:     60x20 2.0 us, 97x41 2.5, 59x100 3.0
+//   cooperative: 151x49 3.5, 200x100 4.3, 400x200 6.8 (17 before), 460x270 8.5 (19)
+// Two groups are the line because from three on a cluster CTA has more than 320
+// threads, which hold fewer registers (96, with spills of 200-408 bytes), and its
+// groups share an SM of which the cooperative form has 148: cluster / cooperative
+// with one group a CTA 2.5 / 3.6 us (97x41), two 3.0 / 3.6 (59x100), three 3.6 / 3.5
+// (151x49), 3.4 / 3.3 (375x25) and 4.2 / 3.7 (80x100), four 5.0 / 3.7 (96x96).
 struct ResPlan {
   int L = 0, groups = 0, units = 0, per_cta = 0;
   bool cluster = false;
@@ -932,7 +937,7 @@ template <int PRE> ResPlan res_plan(const tpo_grid *g, int cluster_ctas) {
   if (p.units > RES_MAX_UNITS) return p;
   const int most = std::min(RES_GROUPS, RES_MAX_THREADS / (res_warps(p.L) * 32));
   for (const bool cluster : {true, false})
-    for (int m = 1; m <= (cluster ? std::min(most, 2) : most) && !p; ++m)
+    for (int m = 1; m <= (cluster ? std::min(most, RES_CLUSTER_GROUPS) : most) && !p; ++m)
       if ((p.units + m - 1) / m <= (cluster ? cluster_ctas : sm_count())) {
         p.per_cta = m;
         p.cluster = cluster;

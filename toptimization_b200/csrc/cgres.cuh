@@ -1,7 +1,8 @@
 // A whole plain-FP64 solve in one launch, for grids whose PCG state fits on the
-// chip: two nodes per thread, at most one CTA per SM (about 140,000 nodes, 2D,
-// point preconditioners); one thread-block cluster where 16 CTAs hold the grid
-// (about 14,000 nodes), a cooperative launch otherwise.
+// chip: two nodes per thread, at most one CTA per SM (2D, point preconditioners;
+// 592 groups of 30 rows by 8 columns, 142,080 nodes where the grid fills them, 124,881
+// at 460x270); one thread-block cluster where 16 CTAs hold the grid (32 groups, 7,680
+// nodes at most), a cooperative launch otherwise.
 //
 // On such a grid the one-launch-per-iteration form (k_cgstep) spends 14-16 us
 // an iteration on latency: launch, filling the TMA ring, eleven columns one
@@ -64,6 +65,7 @@ constexpr int RES_RED_THREADS = 160;  // threads of the CTA whose summation orde
 constexpr int RES_MAX_THREADS = 640;
 constexpr int RES_MAX_UNITS = 592;    // groups: their sums lie in shared memory
 constexpr int RES_CLUSTER_CTAS = 16;  // non-portable cluster size
+constexpr int RES_CLUSTER_GROUPS = 2; // groups of a cluster's CTA at most
 constexpr int RES_COPIES = 16;
 constexpr int RES_ALL_UNITS = 160, RES_LEADERS = 8;
 constexpr int RES_SMEM_MAX = 112 * 1024;  // dynamic: 160 B a thread at most

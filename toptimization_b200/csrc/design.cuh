@@ -104,6 +104,8 @@ __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
 // whose box lies inside the grid takes the weight sum den_in (filter_den).
 // Values and weights are added in the reference's order (dx, then dy). At rmin = 4
 // on 2048x1024 elements 96 -> 33 us (46 us with the tile staged one load at a time).
+// F_SENS keeps the tile's own rho from the staging: its last division read it again
+// lane by column, a third of the time at R = 1 (29.1 -> 20.7 us; R = 4 39.7 -> 32.9).
 constexpr int F_ROWS = 8;
 static_assert(F_THREADS / 32 * F_ROWS == FT, "a CTA covers the tile");
 template <int MODE, int R>
@@ -354,7 +356,8 @@ __global__ void __launch_bounds__(S_THREADS, 5)
 //   rise) a pass evaluates the three next levels of the bisection tree, the
 //   seven midpoints the next three steps can visit, and walks it.
 // The midpoints, their order, the stop test and the step count are those of
-// the one-at-a-time bisection. About 7 passes instead of 50.
+// the one-at-a-time bisection. At most 7 passes instead of 50; with dv, where every
+// level is walked, at most 17 (25 on large designs, below).
 // With dv = 1 the candidate is rho sqrt(-dc / (lambda + 1e-20)), so a pass needs
 // s = rho sqrt(-dc) once and then a multiplication by 1 / sqrt(lambda + 1e-20),
 // two comparisons and an addition per lambda. (1e-20 is not lost beside lambda:

@@ -19,8 +19,8 @@ Preconditioners: "jacobi", "block_jacobi" (the reference's element-block
 form), "nodal_block_jacobi" (2x2 nodal blocks, new) and "none".
 Recurrence: "auto" (one kernel launch per iteration, in the Chronopoulos-Gear
 form with a single global reduction, for the plain FP64 solve with a point
-preconditioner, and one for the whole solve on grids of up to about 140,000
-nodes; the element-block preconditioner and the mixed form keep two),
+preconditioner, and one for the whole solve on grids that fit the chip, 142,080
+nodes at most; the element-block preconditioner and the mixed form keep two),
 "standard" (the reference's own recurrence, two launches per iteration) or
 "single" (force the one-launch form). The two recurrences produce the same
 iterates in exact arithmetic.
