@@ -24,12 +24,21 @@ constexpr int F_MAXR = 16;
 
 enum FilterMode { F_DENSITY = 0, F_SENS = 1 };
 
+// largest |dy| with a positive weight beside |dx| (-1: none)
+__device__ __forceinline__ int filter_chord(double rmin, int dx, int R) {
+  int m = -1;
+  for (int dy = 0; dy <= R; ++dy)
+    if (rmin - sqrt((double)(dx * dx + dy * dy)) > 0.0) m = dy;
+  return m;
+}
+
 // Radii from F_REGR + 1 to F_MAXR. (bx, by) = (tile row, tile column) of this CTA.
-// Bound by two shared loads and two tests per neighbour and by the warps that cover
-// their latency: a tile of 21 to 41 KB limits the CTAs of an SM, so a CTA has 256
-// threads, in a kernel without the register form's 78 registers. Density filter of
-// 517x173 elements at R = 9, 12, 16: 40, 61, 96 us (47, 67, 105 without the unrolled
-// row; 80, 114, 179 with 128 threads and both forms in one kernel).
+// Bound by two shared loads per neighbour and by the warps that cover their latency:
+// a tile of 21 to 41 KB limits the CTAs of an SM, so a CTA has 256 threads, in a
+// kernel without the register form's 78 registers. A row of the box is its chord of
+// positive weights inside the grid, without a test per neighbour. Density filter of
+// 517x173 elements at R = 9, 12, 16: 36, 51, 78 us (47, 67, 105 with the tests; 80,
+// 114, 179 with 128 threads and both forms in one kernel).
 template <int MODE>
 __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
                                            const double *__restrict__ x,
@@ -42,8 +51,10 @@ __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
   const int TW = FT + 2 * R;  // staged tile edge
   double *wt = fsm;           // W*W weights
   double *tile = fsm + W * W; // TW*TW values, index tx*TW + ty
+  __shared__ int chord[F_MAXR + 1];  // largest |dy| with a positive weight (-1: none)
   const int ex0 = by * FT, ey0 = bx * FT;
 
+  if (threadIdx.x <= R) chord[threadIdx.x] = filter_chord(rmin, threadIdx.x, R);
   for (int k = threadIdx.x; k < W * W; k += blockDim.x) {
     const int dx = k / W - R, dy = k % W - R;
     wt[k] = rmin - sqrt((double)(dx * dx + dy * dy));
@@ -71,14 +82,12 @@ __device__ __forceinline__ void filter_any(int nx, int ny, double rmin, int R,
       if (jx < 0 || jx >= nx) continue;
       const double *trow = tile + (size_t)(tx + R + dx) * TW + (ty + R);
       const double *wrow = wt + (dx + R) * W + R;
+      const int m = chord[abs(dx)], d1 = min(m, ny - 1 - ey);
 #pragma unroll 4
-      for (int dy = -R; dy <= R; ++dy) {
+      for (int dy = max(-m, -ey); dy <= d1; ++dy) {
         const double w = wrow[dy];
-        const int jy = ey + dy;
-        if (w > 0.0 && jy >= 0 && jy < ny) {
-          num = fma(w, trow[dy], num);
-          den += w;
-        }
+        num = fma(w, trow[dy], num);
+        den += w;
       }
     }
     const size_t e = (size_t)ex * ny + ey;
@@ -128,12 +137,7 @@ __device__ __forceinline__ void filter_reg(int nx, int ny, double rmin,
     const int dx = k / (R + 1), dy = k % (R + 1);
     wt[k] = rmin - sqrt((double)(dx * dx + dy * dy));
   }
-  if (threadIdx.x <= R) {
-    int m = -1;
-    for (int dy = 0; dy <= R; ++dy)
-      if (rmin - sqrt((double)(threadIdx.x * threadIdx.x + dy * dy)) > 0.0) m = dy;
-    chord[threadIdx.x] = m;
-  }
+  if (threadIdx.x <= R) chord[threadIdx.x] = filter_chord(rmin, threadIdx.x, R);
   constexpr int NB = 8;  // loads in flight per thread
   for (int k0 = threadIdx.x; k0 < TC * TH; k0 += NB * F_THREADS) {
     double v[NB], q[MODE == F_SENS ? NB : 1];
