@@ -10,21 +10,21 @@ from conftest import REPO
 SRC = (REPO / "toptimization_b200" / "csrc" / "cgres.cuh").read_text()
 
 
-def _buffers():
-    """Copies of {alpha, beta, go on} in a CTA's shared memory."""
-    m = re.search(r"__shared__ double s_ab(?:\[(\d+)\])?\[3\]", SRC)
-    return int(m.group(1) or 1)
-
-
 def test_coefficients_wait_for_every_warp_that_reads_them():
     """A CTA that does not collect the sums itself, with one group of nodes and
     one empty group. A warp of the first publishes its sums of exchange e, gets
     that exchange's coefficients (they come after its sums) and writes them for
     the CTA; both meet at a barrier and read them. The empty group publishes
-    nothing, so nothing but the buffers keeps the next exchange's coefficients
-    from a read that is late."""
-    last, copies = 5, _buffers()
-    # steps of the writer: 3 (e - 1) + (write, barrier, read); of the reader: 2 (e - 1) + (barrier, read)
+    nothing, so a late read of it has to be kept from the next exchange's
+    coefficients otherwise: by a barrier after the reads, or by a second buffer."""
+    m = re.search(r"__shared__ double s_ab(?:\[(\d+)\])?\[3\]", SRC)
+    copies = int(m.group(1) or 1)
+    reads = SRC.index("alpha = s_ab[0];") if copies == 1 else 0
+    held = re.search(r"if \(!lead && unfilled\) __syncthreads\(\);", SRC[reads:]) is not None
+    last = 5
+    after = ["barrier"] if held else []
+    writer = [(op, e) for e in range(1, last + 1) for op in ["write", "barrier", "read"] + after]
+    reader = [(op, e) for e in range(1, last + 1) for op in ["barrier", "read"] + after]
     seen, todo = set(), [(0, 0, (0,) * copies)]
     while todo:
         state = todo.pop()
@@ -32,18 +32,20 @@ def test_coefficients_wait_for_every_warp_that_reads_them():
             continue
         seen.add(state)
         w, r, buf = state
-        we, ws, re_, rs = w // 3 + 1, w % 3, r // 2 + 1, r % 2
-        if we <= last and ws == 0:
+        wop, we = writer[w] if w < len(writer) else (None, 0)
+        rop, re_ = reader[r] if r < len(reader) else (None, 0)
+        if wop == "write":
             todo.append((w + 1, r, tuple(we if i == we % copies else b for i, b in enumerate(buf))))
-        if we <= last and ws == 2:
+        elif wop == "read":
             assert buf[we % copies] == we
             todo.append((w + 1, r, buf))
-        if we <= last and ws == 1 and rs == 0 and re_ == we:  # both at the barrier
+        elif wop == "barrier" and rop == "barrier":
+            assert we == re_
             todo.append((w + 1, r + 1, buf))
-        if re_ <= last and rs == 1:
+        if rop == "read":
             assert buf[re_ % copies] == re_, "a warp reads the coefficients of a later exchange"
             todo.append((w, r + 1, buf))
-    assert any(w == 3 * last and r == 2 * last for w, r, _ in seen)
+    assert any(w == len(writer) and r == len(reader) for w, r, _ in seen)
 
 
 def _element_bytes(fn):

@@ -151,10 +151,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_cgres(ResArgs A) {
   extern __shared__ __align__(16) double res_sm[];
   __shared__ double s_sum[CLUSTER ? 2 : 1][3][CLUSTER ? RES_GROUPS : RES_MAX_UNITS];
   __shared__ double s_red[3][RES_RED_THREADS / 32];
-  // alpha, beta, 1 if another iteration follows, by parity of the exchange: in a CTA that
-  // does not collect the sums nothing else orders an empty group's reads before the next
-  // exchange's writes
-  __shared__ double s_ab[2][3];
+  __shared__ double s_ab[3];  // alpha, beta, 1 if another iteration follows
   const int nx = A.nx, ny = A.ny, ny1 = ny + 1, L = A.L, U = A.units;
   const int W = res_warps(L), C = 2 * W;            // warps, columns of a group
   const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
@@ -270,6 +267,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_cgres(ResArgs A) {
   // group, held by its warps 0 .. 2; collect the halo nodes' values and all
   // sums in s_sum. False in every thread when a wait ran out (cooperative form).
   const bool lead = CLUSTER || A.leaders == 0 || cta < A.leaders;
+  const bool unfilled = !CLUSTER && (cta + 1) * A.per_cta > U;  // the last CTA may have empty groups
   const int copies = A.leaders ? A.leaders : RES_COPIES;
   uint32_t epoch = 0;
   double rz = 0.0, alpha = 0.0, inv_rz = 0.0, inv_alpha = 0.0;
@@ -313,7 +311,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_cgres(ResArgs A) {
     } else {
       const int from = cta % copies, words = with_sums ? (lead ? 3 * U : 3) : 0;
       const double *src = lead ? sums + (size_t)from * 6 * U : A.coef + (b * copies + from) * 6;
-      double *to = lead ? &s_sum[0][0][0] : s_ab[b];  // s_sum: [3][units]
+      double *to = lead ? &s_sum[0][0][0] : s_ab;  // s_sum: [3][units]
       bool need[2] = {halo[0], halo[1]}, ok = true;
       int k = t;  // next word this thread collects
       for (int i = 0; need[0] || need[1] || k < words; ++i) {
@@ -479,19 +477,23 @@ __global__ void __launch_bounds__(THREADS, 1) k_cgres(ResArgs A) {
       rz = gamma;
       const double go = status == TPO_SOLVE_RUNNING && it < max_iter ? 1.0 : 0.0;
       if (lane == 0) {
-        s_ab[epoch & 1][0] = al;
-        s_ab[epoch & 1][1] = b;
-        s_ab[epoch & 1][2] = go;
+        s_ab[0] = al;
+        s_ab[1] = b;
+        s_ab[2] = go;
       }
       if (!CLUSTER && A.leaders && lane < 3)
         ll_store(A.coef, ((epoch & 1) * A.leaders + cta) * 3 + lane,
                  lane == 0 ? al : lane == 1 ? b : go, epoch);
     }
     if (lead) __syncthreads();
-    const double *ab = s_ab[epoch & 1];
-    alpha = ab[0];
-    beta = ab[1];
-    if (ab[2] == 0.0) break;
+    alpha = s_ab[0];
+    beta = s_ab[1];
+    const bool go_on = s_ab[2] != 0.0;
+    // In a CTA that does not collect the sums, the next exchange writes s_ab without
+    // a barrier. Its groups' own sums hold that back until all their warps have read;
+    // an empty group has none. (Two buffers instead cost every CTA 3 % at 400x200.)
+    if (!lead && unfilled) __syncthreads();
+    if (!go_on) break;
     init = false;
   }
 #pragma unroll
